@@ -3,24 +3,37 @@
 // GLRT (shp/_glrt.py:13-130): the Rayleigh scale^2 = (var + mean^2)/2 is written to a
 // pitched buffer, and each CTA stages its input region into shared memory with one
 // TMA tiled copy (cp.async.bulk.tensor.2d, completion on an mbarrier with a bounded
-// wait).  log(scale^2) is taken once per staged sample; each (pixel, offset) test
-// needs one more log, of the pooled scale.  Window starts follow lax.dynamic_slice
-// (clamped into the image: windows shift at the edges), validity follows the
-// unclamped origin and the window centre is always False -- the reference's
-// semantics.  The statistic is the reference's float32 expression
-// nslc * (2*log(pooled) - log(s1) - log(s2)) without FMA contraction; its three logs
-// cancel, so its rounding is a few 1e-6 of the cutoff.  Where it lands within 1e-5
-// (relative) of the cutoff, the decision is taken on the same statistic evaluated in
-// double precision as nslc * log1p((s1 - s2)^2 / (4 s1 s2)) (algebraically equal, no
-// cancellation), so every mask bit is the exact comparison on the float32 scale^2.
+// wait).  Window starts follow lax.dynamic_slice (clamped into the image: windows shift
+// at the edges), validity follows the unclamped origin and the window centre is always
+// False -- the reference's semantics.  The reference's float32 statistic
+// nslc * (2*log(pooled) - log(s1) - log(s2)) < threshold is, exactly,
+//     (s1 + s2)^2 < 4 exp(threshold / nslc) s1 s2,
+// which needs no logarithm: five float32 operations per (pixel, offset).  They carry
+// less than 5e-7 of relative error; where the two sides are within 2e-6 of each other,
+// the decision is taken in double precision on nslc * log1p((s1 - s2)^2 / (4 s1 s2))
+// (algebraically equal, no cancellation), so every mask bit is the exact comparison on
+// the float32 scale^2.  Scales whose products would overflow float32 and thresholds
+// outside the usual range take the statistic with its logarithms (glrt_test), refined
+// in the same way where its rounding could reach the cutoff.
 //
-// KS (shp/_ks.py:22-239): amplitudes are sorted per pixel (NaN last, like np.sort);
-// each (pixel, neighbour) pair walks the two-sample merge exactly as
-// _get_max_cdf_dist does.  The reference accumulates the ECDFs by repeated float64
-// additions of 1/n, so after i steps an ECDF equals T[i] (the i-fold sum); the walk
-// only needs the integer positions and a host-built table of the admissible
-// partner range {i2 : |T[i1] - T[i2]| < cutoff}, an interval because T increases.
-// The decision is therefore bit-identical to the float64 walk.
+// KS (shp/_ks.py:22-239): amplitudes are sorted per pixel (NaN last, like np.sort).  The
+// reference walks the two-sample merge of each (pixel, neighbour) pair and rejects it
+// where the ECDFs come apart by the cutoff.  It accumulates the ECDFs by repeated
+// float64 additions of 1/n, so after i steps an ECDF equals T[i] (the i-fold sum) and a
+// walk position (i1, i2) is admissible where i2 lies in the interval
+// {i2 : |T[i1] - T[i2]| < cutoff}, T being increasing.  Without ties the walk leaves the
+// band exactly where some sample of the neighbour lies outside its envelope,
+//     lo_t < x2[t] < hi_t,  lo_t = x1[m(t) - 1],  hi_t = x1[min {i : m(i) - 1 = t}],
+// with m(t) the smallest i1 that admits i2 = t + 1: x2[t] is taken before x1[m(t) - 1]
+// when it is smaller, and the lower bound is the same statement with the two series
+// exchanged.  A violated bound rejects, all bounds strictly met accept, and only a pair
+// with an equality (a tie decides by the walk's order) or with a non-finite sample is
+// walked step by step.  The decision is therefore bit-identical to the float64 walk.
+//
+// Both kernels gather a window row's decisions as bits, one item per (pixel, window
+// row, 32 offsets) with consecutive pixels on consecutive lanes (conflict-free reads of
+// the staged tile), and write the mask bytes of each output row afterwards, four per
+// store.
 #include <cuda.h>
 
 #include <algorithm>
@@ -87,22 +100,78 @@ __global__ void k_glrt_scale(const float* __restrict__ mean, const float* __rest
     scale2[r * pitch + c] = fdiv(fadd(var[i], fmul(m, m)), 2.f);
 }
 
-// One (pixel, offset) test: threshold > statistic, the float32 statistic refined in
-// double precision near the cutoff (see above).  NaN statistics stay False.
-__device__ __forceinline__ bool glrt_test(float s1, float s2, float l1, float l2, float nslc, float thr) {
+// threshold > statistic in double precision on the float32 scales
+__device__ __noinline__ bool glrt_exact(float s1, float s2, float nslc, float thr) {
+    const double d = (double)s1 - (double)s2;
+    const double t = (double)nslc * log1p(d * d / (4.0 * (double)s1 * (double)s2));
+    return (double)thr > t;
+}
+
+// One (pixel, offset) test with the float32 statistic, refined in double precision near
+// the cutoff (see above).  NaN statistics stay False.
+__device__ __noinline__ bool glrt_test(float s1, float s2, float nslc, float thr) {
     // (s1 + s2) / 2 == (s1 + s2) * 0.5 exactly in IEEE arithmetic
     const float pooled = fmul(fadd(s1, s2), 0.5f);
-    const float stat = fmul(nslc, fsub(fsub(fmul(2.f, logf(pooled)), l1), l2));
+    const float lp = fmul(2.f, logf(pooled)), l1 = logf(s1), l2 = logf(s2);
+    const float stat = fmul(nslc, fsub(fsub(lp, l1), l2));
     bool shp = thr > stat;
-    if (fabsf(stat - thr) <= 1e-5f * thr) {
-        const double d = (double)s1 - (double)s2;
-        const double t = (double)nslc * log1p(d * d / (4.0 * (double)s1 * (double)s2));
-        shp = (double)thr > t;
-    }
+    // the rounding of the three logarithms and of their cancelling sum
+    const float err = nslc * 3e-7f * (fabsf(lp) + fabsf(l1) + fabsf(l2));
+    if (fabsf(stat - thr) <= fmaf(1e-5f, thr, err)) shp = glrt_exact(s1, s2, nslc, thr);
     return shp;
 }
 
-template <bool kBits>
+// Bytes (0/1) of an output row's masks from their bits: window row r (pixel by pixel) of
+// the tile row has its wx bits in the nw words at bits + r * nw, zero beyond wx; the
+// bytes go to dst[0 .. rows * wx).  C bytes (4, 8 or 16, at most wx + 1, so that they
+// touch two window rows at most) per aligned store.
+template <int C>
+__device__ __forceinline__ void write_masks(uint8_t* dst, const uint32_t* bits, int rows, int wx, int nw) {
+    const int len = rows * wx;
+    const int head = min(len, (int)((C - (uint32_t)(reinterpret_cast<uintptr_t>(dst) & (C - 1))) & (C - 1)));
+    const int chunks = (len - head) / C, tail = head + C * chunks;
+    auto bit = [&](int k) -> uint32_t {
+        const int r = k / wx, wb = k - r * wx;
+        return (bits[r * nw + (wb >> 5)] >> (wb & 31)) & 1u;
+    };
+    const float inv_wx = 1.f / (float)wx;
+    for (int q = threadIdx.x; q < chunks; q += blockDim.x) {
+        const int k = head + C * q;
+        int r = (int)((float)k * inv_wx);  // k / wx: the float quotient is off by one at most
+        int wb = k - r * wx;
+        if (wb < 0) {
+            --r;
+            wb += wx;
+        } else if (wb >= wx) {
+            ++r;
+            wb -= wx;
+        }
+        const uint32_t* w = bits + r * nw + (wb >> 5);
+        const int sh = wb & 31, left = wx - wb;
+        uint32_t v = w[0] >> sh;
+        if (sh > 32 - C && left > 32 - sh) v |= w[1] << (32 - sh);  // into the row's next word
+        if (left < C) v |= bits[(r + 1) * nw] << left;              // into the next window row
+        uint32_t o[C / 4];
+#pragma unroll
+        for (int i = 0; i < C / 4; ++i) o[i] = (((v >> (4 * i)) & 0xfu) * 0x00204081u) & 0x01010101u;
+        if constexpr (C == 16) *reinterpret_cast<uint4*>(dst + k) = make_uint4(o[0], o[1], o[2], o[3]);
+        else if constexpr (C == 8) *reinterpret_cast<uint2*>(dst + k) = make_uint2(o[0], o[1]);
+        else *reinterpret_cast<uint32_t*>(dst + k) = o[0];
+    }
+    if ((int)threadIdx.x < head) dst[threadIdx.x] = (uint8_t)bit(threadIdx.x);
+    if ((int)threadIdx.x < len - tail) dst[tail + threadIdx.x] = (uint8_t)bit(tail + threadIdx.x);
+}
+
+__device__ __forceinline__ void write_mask_row(uint8_t* dst, const uint32_t* bits, int rows, int wx, int nw) {
+    if (wx >= 15) write_masks<16>(dst, bits, rows, wx, nw);
+    else if (wx >= 7) write_masks<8>(dst, bits, rows, wx, nw);
+    else if (wx >= 3) write_masks<4>(dst, bits, rows, wx, nw);
+    else
+        for (int k = threadIdx.x; k < rows; k += blockDim.x) dst[k] = (uint8_t)(bits[k] & 1u);  // wx == 1
+}
+
+// Issue-bound.  1024 x 2048 pixels, 11 x 23 windows: 346 us (1.53 TB/s of mask bytes); a
+// logarithm per test and one byte per thread in the writes took 1098 us.
 __global__ void __launch_bounds__(256) k_glrt(const __grid_constant__ CUtensorMap tmap, GlrtArgs a) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
@@ -111,8 +180,8 @@ __global__ void __launch_bounds__(256) k_glrt(const __grid_constant__ CUtensorMa
     const uint32_t mis = (uint32_t)__cvta_generic_to_shared(smem_raw) & 127u;
     float* raw = reinterpret_cast<float*>(smem_raw + ((128u - mis) & 127u));
     const int n_tile = a.box_w * a.box_h;
-    float* lg = raw + n_tile;
-    const int wy = 2 * a.hy + 1, wx = 2 * a.hx + 1;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(raw + n_tile);  // [pixel][window row][nw]
+    const int wy = 2 * a.hy + 1, wx = 2 * a.hx + 1, nw = (wx + 31) >> 5;
     const int or0 = blockIdx.y * a.tile_r, oc0 = blockIdx.x * a.tile_c;
     const int or1 = min(or0 + a.tile_r, a.out_rows), oc1 = min(oc0 + a.tile_c, a.out_cols);
     const int rr0 = clamp_start(a.sy / 2 + or0 * a.sy, a.hy, wy, a.rows);
@@ -144,79 +213,74 @@ __global__ void __launch_bounds__(256) k_glrt(const __grid_constant__ CUtensorMa
         __syncthreads();
         return;
     }
-    for (int i = threadIdx.x; i < n_tile; i += blockDim.x) lg[i] = logf(raw[i]);
-    __syncthreads();
+    // a negative scale has a NaN logarithm: never an SHP.  Finite scales above the
+    // bound (their products overflow) send the tile to the logarithms.
+    bool large = !a.ratio;
+    for (int i = threadIdx.x; i < n_tile; i += blockDim.x) {
+        const float v = raw[i];
+        if (v < 0.f) raw[i] = nanf("");
+        large |= v > a.ratio_max && v < INFINITY;
+    }
+    const bool use_log = __syncthreads_or(large);
 
     const float nslc = (float)a.nslc;
-    const int W = wy * wx;
-    if (!kBits) {
-        // per output row of the tile: one item per (pixel, window row) computes the
-        // row's wx bytes into shared memory (index arithmetic once per item, the valid
-        // column range hoisted), then the row's contiguous segment of the output is
-        // written with consecutive bytes per consecutive threads (coalesced)
-        uint8_t* ob = reinterpret_cast<uint8_t*>(lg + n_tile);
-        const int tc = oc1 - oc0;
-        for (int orow = or0; orow < or1; ++orow) {
-            const int in_r = a.sy / 2 + orow * a.sy;
-            const int r0 = clamp_start(in_r, a.hy, wy, a.rows);
-            const int ur0 = in_r - a.hy;
-            for (int it = threadIdx.x; it < tc * wy; it += blockDim.x) {
-                const int pix = it / wy, wa = it - pix * wy;
-                const int in_c = a.sx / 2 + (oc0 + pix) * a.sx;
-                const int c0 = clamp_start(in_c, a.hx, wx, a.cols);
-                const int uc0 = in_c - a.hx;
-                uint8_t* dst = ob + pix * W + wa * wx;
-                const bool row_ok = (wa >= -ur0) && (wa < a.rows - ur0);
-                // valid window columns of the unclamped origin
-                const int wb0 = row_ok ? max(0, -uc0) : wx, wb1 = row_ok ? min(wx, a.cols - uc0) : wx;
-                const int i1 = (in_r - rr0) * a.box_w + (in_c - x0);
-                const float s1 = raw[i1], l1 = lg[i1];
-                const float* rraw = raw + (r0 + wa - rr0) * a.box_w + (c0 - x0);
-                const float* rlg = lg + (r0 + wa - rr0) * a.box_w + (c0 - x0);
-                for (int wb = 0; wb < wx; ++wb) {
-                    bool shp = false;
-                    if (wb >= wb0 && wb < wb1 && !(wa == a.hy && wb == a.hx))
-                        shp = glrt_test(s1, rraw[wb], l1, rlg[wb], nslc, a.thr);
-                    dst[wb] = shp ? 1 : 0;
-                }
+    const int tc = oc1 - oc0, npix = (or1 - or0) * tc;
+    const int items = npix * wy * nw;
+    for (int it = threadIdx.x; it < items; it += blockDim.x) {
+        const int rest = it / npix, pix = it - rest * npix;
+        const int word = rest / wy, wa = rest - word * wy;
+        const int pr = pix / tc;
+        const int in_r = a.sy / 2 + (or0 + pr) * a.sy, in_c = a.sx / 2 + (oc0 + pix - pr * tc) * a.sx;
+        const int r0 = clamp_start(in_r, a.hy, wy, a.rows), c0 = clamp_start(in_c, a.hx, wx, a.cols);
+        const int ur0 = in_r - a.hy, uc0 = in_c - a.hx;
+        // valid window columns of the unclamped origin, within this word
+        const bool row_ok = (wa >= -ur0) && (wa < a.rows - ur0);
+        const int b0 = 32 * word, nb = min(wx - b0, 32);
+        const int v0 = max(max(0, -uc0) - b0, 0), v1 = row_ok ? min(min(wx, a.cols - uc0) - b0, nb) : 0;
+        uint32_t valid = v1 > v0 ? (v1 - v0 == 32 ? 0xffffffffu : ((1u << (v1 - v0)) - 1u) << v0) : 0u;
+        if (wa == a.hy && a.hx >= b0 && a.hx < b0 + 32) valid &= ~(1u << (a.hx - b0));
+        const float s1 = raw[(in_r - rr0) * a.box_w + (in_c - x0)];
+        const float* row = raw + (r0 + wa - rr0) * a.box_w + (c0 - x0) + b0;
+        uint32_t shp = 0u, close = 0u;
+        if (!use_log) {
+            const float k1 = a.four_c * s1;
+            // each decision is the sign of a difference, shifted into a word (first offset
+            // highest); NaN differences are positive (canonical NaN)
+            auto test = [&](int wb) {
+                const float s2 = row[wb];
+                const float sum = s1 + s2;
+                const float r = k1 * s2;
+                const float diff = fmaf(sum, sum, -r);
+                // 1e-40 covers products that lose bits below the normal range
+                const float margin = fabsf(diff) - fmaf(2e-6f, r, 1e-40f);
+                shp = __funnelshift_l(__float_as_uint(diff), shp, 1);
+                close = __funnelshift_l(__float_as_uint(margin), close, 1);
+            };
+            int wb = 0;
+            for (; wb + 8 <= nb; wb += 8) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) test(wb + i);
             }
-            __syncthreads();
-            const int64_t seg0 = ((int64_t)orow * a.out_cols + oc0) * W;
-            for (int k = threadIdx.x; k < tc * W; k += blockDim.x) a.is_shp[seg0 + k] = ob[k];
-            __syncthreads();
-        }
-    } else {
-        // one window row (<= 64 offsets) per iteration, packed into words_per_row words
-        const int tc = oc1 - oc0;
-        const int items = (or1 - or0) * tc * wy;
-        for (int it = threadIdx.x; it < items; it += blockDim.x) {
-            const int wa = it % wy;
-            const int pix = it / wy;
-            const int orow = or0 + pix / tc, ocol = oc0 + pix % tc;
-            const int in_r = a.sy / 2 + orow * a.sy, in_c = a.sx / 2 + ocol * a.sx;
-            const int r0 = clamp_start(in_r, a.hy, wy, a.rows), c0 = clamp_start(in_c, a.hx, wx, a.cols);
-            const int ur0 = in_r - a.hy, uc0 = in_c - a.hx;
-            const bool row_ok = (wa >= -ur0) && (wa < a.rows - ur0);
-            const int i1 = (in_r - rr0) * a.box_w + (in_c - x0);
-            const float s1 = raw[i1], l1 = lg[i1];
-            uint32_t w0 = 0, w1 = 0;
-            if (row_ok) {
-                const float* rraw = raw + (r0 + wa - rr0) * a.box_w + (c0 - x0);
-                const float* rlg = lg + (r0 + wa - rr0) * a.box_w + (c0 - x0);
-                for (int wb = 0; wb < wx; ++wb) {
-                    const bool valid = (wb >= -uc0) && (wb < a.cols - uc0) && !(wa == a.hy && wb == a.hx);
-                    if (!valid) continue;
-                    if (glrt_test(s1, rraw[wb], l1, rlg[wb], nslc, a.thr)) {
-                        if (wb < 32) w0 |= 1u << wb;
-                        else w1 |= 1u << (wb - 32);
-                    }
-                }
+#pragma unroll 1
+            for (; wb < nb; ++wb) test(wb);
+            shp = __brev(shp) >> (32 - nb);
+            close = __brev(close) >> (32 - nb);
+            close &= valid;
+            while (close) {
+                const int wb2 = __ffs(close) - 1;
+                close &= close - 1u;
+                shp = (shp & ~(1u << wb2)) | (uint32_t)glrt_exact(s1, row[wb2], nslc, a.thr) << wb2;
             }
-            uint32_t* dst = a.bits + (((int64_t)orow * a.out_cols + ocol) * wy + wa) * a.words_per_row;
-            dst[0] = w0;
-            if (a.words_per_row > 1) dst[1] = w1;
+        } else {
+            for (int wb = 0; wb < nb; ++wb)
+                if ((valid >> wb) & 1u) shp |= (uint32_t)glrt_test(s1, row[wb], nslc, a.thr) << wb;
         }
+        bits[(pix * wy + wa) * nw + word] = shp & valid;
     }
+    __syncthreads();
+    for (int orow = or0; orow < or1; ++orow)
+        write_mask_row(a.is_shp + ((int64_t)orow * a.out_cols + oc0) * (wy * wx), bits + (orow - or0) * tc * wy * nw,
+                       tc * wy, wx, nw);
 }
 
 // ---------------------------------------------------------------------------------
@@ -252,18 +316,40 @@ __global__ void __launch_bounds__(128) k_sort_pixels(const float* __restrict__ i
         if (t < n) out[(int64_t)t * npix + p] = v[t];
 }
 
-__global__ void __launch_bounds__(256) k_ks(KsArgs a) {
-    extern __shared__ float ks_smem[];
-    // layout: lo[n+1], hi[n+1] (int), then the staged sorted samples [region][n]
-    int* lo = reinterpret_cast<int*>(ks_smem);
-    int* hi = lo + (a.n + 1);
-    float* samp = reinterpret_cast<float*>(hi + (a.n + 1));
-    const int n = a.n;
-    for (int i = threadIdx.x; i <= n; i += blockDim.x) {
-        lo[i] = a.lo[i];
-        hi[i] = a.hi[i];
+// The reference's merge walk of two sorted series.
+__device__ __noinline__ bool ks_walk(const float* x1, const float* x2, int n, const KsArgs& a) {
+    int i1 = 0, i2 = 0;
+    for (int iout = 0; iout < 2 * n;) {
+        if (i1 == n) {
+            ++i2;
+        } else if (i2 == n || x1[i1] < x2[i2]) {
+            ++i1;
+        } else if (x1[i1] > x2[i2]) {
+            ++i2;
+        } else {  // a tie (or a comparison with NaN): both step
+            ++i1;
+            ++i2;
+            ++iout;
+        }
+        ++iout;
+        if (i2 < a.lo[i1] || i2 > a.hi[i1]) return false;
     }
-    const int wy = 2 * a.hy + 1, wx = 2 * a.hx + 1;
+    return true;
+}
+
+// A thread keeps the envelope of its pixel in registers and takes up to 32 neighbours
+// through it.  With d the smallest t that has a lower bound, sample t has an upper bound
+// only for t < n - d, so the bounds pair up: x2[s + d] > low[s], x2[s] < high[s] for
+// s < ns = n - d, NS being ns rounded up to a multiple of 4.  The samples of a pixel are
+// contiguous in shared memory (immediate offsets), at an odd pitch (consecutive pixels
+// fall into different banks).  Issue-bound (63 % of issue slots): 512 x 512 pixels, 20
+// dates, 11 x 23 windows, 300 us; a merge walk per thread, divergent and with bank
+// conflicts, took 3949 us.
+template <int NS>
+__global__ void __launch_bounds__(256) k_ks(const __grid_constant__ KsArgs a) {
+    extern __shared__ float samp[];  // sorted samples [pixel][np], then the mask bits
+    const int n = a.n, np = a.n | 1, d = a.n - a.ns;
+    const int wy = 2 * a.hy + 1, wx = 2 * a.hx + 1, nw = (wx + 31) >> 5;
     const int or0 = blockIdx.y * a.tile_r, oc0 = blockIdx.x * a.tile_c;
     const int or1 = min(or0 + a.tile_r, a.out_rows), oc1 = min(oc0 + a.tile_c, a.out_cols);
     // input region of the (unclamped) windows, intersected with the image
@@ -271,49 +357,74 @@ __global__ void __launch_bounds__(256) k_ks(KsArgs a) {
     const int rr1 = min(a.rows, a.sy / 2 + (or1 - 1) * a.sy + a.hy + 1);
     const int cc1 = min(a.cols, a.sx / 2 + (oc1 - 1) * a.sx + a.hx + 1);
     const int rw = cc1 - cc0, rh = rr1 - rr0;
-    for (int i = threadIdx.x; i < rw * rh * n; i += blockDim.x) {
-        const int pix = i % (rw * rh), t = i / (rw * rh);  // pixel-fastest: coalesced reads
-        const int r = rr0 + pix / rw, c = cc0 + pix % rw;
-        samp[pix * n + t] = a.sorted[((int64_t)t * a.rows + r) * a.cols + c];
+    uint32_t* bits = reinterpret_cast<uint32_t*>(samp + a.off_bits);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int tr = warp; tr < n * rh; tr += 8) {  // one warp per (date, row)
+        const int t = tr / rh, r = tr - t * rh;
+        const float* src = a.sorted + ((int64_t)t * a.rows + rr0 + r) * a.cols + cc0;
+        float* dst = samp + r * rw * np + t;
+        for (int c = lane; c < rw; c += 32)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + c * np)), "l"(src + c)
+                         : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int tc = oc1 - oc0, npix = (or1 - or0) * tc;
+    const int items = npix * wy * nw;
+    for (int it = threadIdx.x; it < items; it += blockDim.x) {
+        const int rest = it / npix, pix = it - rest * npix;
+        const int word = rest / wy, wa = rest - word * wy;
+        const int pr = pix / tc;
+        const int in_r = a.sy / 2 + (or0 + pr) * a.sy, in_c = a.sx / 2 + (oc0 + pix - pr * tc) * a.sx;
+        uint32_t shp = 0u;
+        if (in_r - a.hy >= 0 && in_r + a.hy + 1 <= a.rows && in_c - a.hx >= 0 && in_c + a.hx + 1 <= a.cols) {
+            const float* x1 = samp + ((in_r - rr0) * rw + (in_c - cc0)) * np;
+            float low[NS], high[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                const int il = s < a.ns ? a.env_lo[s + d] : -1, ih = s < a.ns ? a.env_hi[s] : -1;
+                low[s] = il >= 0 ? x1[il] : -INFINITY;
+                high[s] = ih >= 0 ? x1[ih] : INFINITY;
+            }
+            const bool special = !(fabsf(x1[n - 1] - x1[0]) < INFINITY);
+            const int b0 = 32 * word, nb = min(wx - b0, 32);
+            const float* q = samp + ((in_r - a.hy + wa - rr0) * rw + (in_c - a.hx - cc0) + b0) * np;
+#pragma unroll 1
+            for (int wb = 0; wb < nb; ++wb, q += np) {
+                const float* qd = q + d;
+                float f4[4] = {INFINITY, INFINITY, INFINITY, INFINITY};  // four short chains of minima
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    if (s < NS - 3 || s < a.ns) {
+                        f4[2 * (s & 1)] = fminf(f4[2 * (s & 1)], qd[s] - low[s]);
+                        f4[2 * (s & 1) + 1] = fminf(f4[2 * (s & 1) + 1], high[s] - q[s]);
+                    }
+                }
+                const float f = fminf(fminf(f4[0], f4[1]), fminf(f4[2], f4[3]));
+                bool ok = f > 0.f;
+                // an equality, or a sample that is not finite
+                if (f == 0.f || special || !(fabsf(q[n - 1] - q[0]) < INFINITY)) ok = ks_walk(x1, q, n, a);
+                if (ok) shp |= 1u << wb;
+            }
+            if (wa == a.hy && a.hx >= b0 && a.hx < b0 + 32) shp &= ~(1u << (a.hx - b0));
+        }
+        bits[(pix * wy + wa) * nw + word] = shp;
     }
     __syncthreads();
-    const int W = wy * wx;
-    const int tc = oc1 - oc0;
-    const int items = (or1 - or0) * tc * W;
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-        const int off = it % W, pix = it / W;
-        const int orow = or0 + pix / tc, ocol = oc0 + pix % tc;
-        const int in_r = a.sy / 2 + orow * a.sy, in_c = a.sx / 2 + ocol * a.sx;
-        const int wa = off / wx, wb = off - wa * wx;
-        bool shp = false;
-        const bool full = in_r - a.hy >= 0 && in_r + a.hy + 1 <= a.rows && in_c - a.hx >= 0 &&
-                          in_c + a.hx + 1 <= a.cols;
-        if (full && !(wa == a.hy && wb == a.hx)) {
-            const float* x1 = samp + ((in_r - rr0) * rw + (in_c - cc0)) * n;
-            const float* x2 = samp + ((in_r - a.hy + wa - rr0) * rw + (in_c - a.hx + wb - cc0)) * n;
-            int i1 = 0, i2 = 0;
-            shp = true;
-            for (int iout = 0; iout < 2 * n;) {
-                if (i1 == n) {
-                    ++i2;
-                } else if (i2 == n || x1[i1] < x2[i2]) {
-                    ++i1;
-                } else if (x1[i1] > x2[i2]) {
-                    ++i2;
-                } else {  // a tie (or a comparison with NaN): both step
-                    ++i1;
-                    ++i2;
-                    ++iout;
-                }
-                ++iout;
-                if (i2 < lo[i1] || i2 > hi[i1]) {
-                    shp = false;
-                    break;
-                }
-            }
-        }
-        a.is_shp[((int64_t)orow * a.out_cols + ocol) * W + off] = shp ? 1 : 0;
+    for (int orow = or0; orow < or1; ++orow)
+        write_mask_row(a.is_shp + ((int64_t)orow * a.out_cols + oc0) * (wy * wx), bits + (orow - or0) * tc * wy * nw,
+                       tc * wy, wx, nw);
+}
+
+template <int NS>
+static dpl_status launch_ks(const KsArgs& a, dim3 grid, size_t smem, cudaStream_t s) {
+    if constexpr (NS <= kMaxNslc) {
+        if (a.ns > NS) return launch_ks<NS + 4>(a, grid, smem, s);
+        DPL_CUDA_TRY(cudaFuncSetAttribute(k_ks<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_ks<NS><<<grid, 256, smem, s>>>(a);
+        return check_launch("k_ks");
     }
+    return fail(DPL_ERR_UNSUPPORTED, "dpl_shp_ks: nslc > 64");
 }
 
 // ---------------------------------------------------------------------------------
@@ -343,11 +454,10 @@ size_t glrt_workspace_size(int64_t rows, int64_t cols) {
 }
 
 dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_t cols, int hy, int hx, int sy,
-                       int sx, int nslc, float threshold, uint8_t* is_shp, uint32_t* bits, int* status,
-                       float* scale2, cudaStream_t s) {
+                       int sx, int nslc, float threshold, uint8_t* is_shp, int* status, float* scale2,
+                       cudaStream_t s) {
     const int wy = 2 * hy + 1, wx = 2 * hx + 1;
     if (wy > rows || wx > cols) return fail(DPL_ERR_INVALID_ARGUMENT, "GLRT window larger than the image");
-    if (bits && wx > 64) return fail(DPL_ERR_UNSUPPORTED, "packed GLRT masks need 2*hx+1 <= 64");
     const int64_t pitch = glrt_pitch(cols);
     const int64_t npix = rows * cols;
     k_glrt_scale<<<ceil_div(npix, 256), 256, 0, s>>>(mean, var, rows, cols, pitch, scale2);
@@ -365,9 +475,14 @@ dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_
     a.nslc = nslc;
     a.thr = threshold;
     a.is_shp = is_shp;
-    a.bits = bits;
-    a.words_per_row = wx > 32 ? 2 : 1;
     a.status = status;
+    // the ratio test: 4 exp(threshold / nslc) in float32, and the largest scale whose
+    // product with it stays finite.  A threshold of 0 (alpha 1) or a ratio beyond 1e12
+    // leaves the float32 range in which the test's error bound holds: logarithms there.
+    const double c = nslc > 0 ? std::exp((double)threshold / nslc) : 0.0;
+    a.ratio = threshold > 0.f && c > 1.0 && c < 1e12;
+    a.four_c = a.ratio ? (float)(4.0 * c) : 0.f;
+    a.ratio_max = a.ratio ? (float)std::sqrt(1e37 / (4.0 * c)) : 0.f;
     if (a.out_rows == 0 || a.out_cols == 0) return DPL_OK;
     // pick the largest tile whose TMA box fits the 256-element box limit and ~96 KB smem
     int tr = 16, tc = 32;
@@ -375,7 +490,12 @@ dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_
     auto box_h = [&](int t) { return (t - 1) * sy + wy; };
     while (tc > 1 && box_w(tc) > 256) tc /= 2;
     while (tr > 1 && box_h(tr) > 256) tr /= 2;
-    while ((size_t)2 * box_w(tc) * box_h(tr) * 4 > 96 * 1024 && (tr > 1 || tc > 1)) {
+    // staged scale^2, then the tile's mask bits
+    auto smem_for = [&](int r, int c) {
+        return (size_t)box_w(c) * box_h(r) * sizeof(float) + 128 +
+               (size_t)r * c * wy * ((wx + 31) / 32) * sizeof(uint32_t);
+    };
+    while (smem_for(tr, tc) > 96 * 1024 && (tr > 1 || tc > 1)) {
         if (tr >= tc && tr > 1) tr /= 2;
         else tc /= 2;
     }
@@ -396,17 +516,11 @@ dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(DPL_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
-    // staged scale^2 and its log, then one output row of byte masks
-    size_t smem = (size_t)2 * a.box_w * a.box_h * sizeof(float) + 128 + (bits ? 0 : (size_t)tc * wy * wx);
+    const size_t smem = smem_for(tr, tc);
     if (smem > (size_t)227 * 1024) return fail(DPL_ERR_UNSUPPORTED, "GLRT window too large for shared memory");
     dim3 grid(ceil_div(a.out_cols, tc), ceil_div(a.out_rows, tr));
-    if (bits) {
-        DPL_CUDA_TRY(cudaFuncSetAttribute(k_glrt<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_glrt<true><<<grid, 256, smem, s>>>(map, a);
-    } else {
-        DPL_CUDA_TRY(cudaFuncSetAttribute(k_glrt<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_glrt<false><<<grid, 256, smem, s>>>(map, a);
-    }
+    DPL_CUDA_TRY(cudaFuncSetAttribute(k_glrt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_glrt<<<grid, 256, smem, s>>>(map, a);
     return check_launch("k_glrt");
 }
 
@@ -430,7 +544,7 @@ extern "C" dpl_status dpl_shp_glrt(const float* mean, const float* var, int64_t 
     int* status = ws.take<int>(64);
     float* scale2 = ws.take<float>((size_t)rows * glrt_pitch(cols));
     DPL_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
-    return launch_glrt(mean, var, rows, cols, hy, hx, sy, sx, nslc, threshold, is_shp, nullptr, status, scale2, s);
+    return launch_glrt(mean, var, rows, cols, hy, hx, sy, sx, nslc, threshold, is_shp, status, scale2, s);
 }
 
 size_t dpl::ks_workspace_size(int64_t nslc, int64_t rows, int64_t cols) {
@@ -473,14 +587,29 @@ extern "C" dpl_status dpl_shp_ks(const float* amp_stack, int64_t nslc, int64_t r
         lo[i1] = l;
         hi[i1] = h;
     }
+    KsArgs a{};
+    for (int i = 0; i <= n; ++i) {
+        a.lo[i] = (int8_t)std::min(lo[i], 127);
+        a.hi[i] = (int8_t)hi[i];
+    }
+    // m(t): the smallest i1 that admits t + 1 neighbour samples; n + 1 if none does (a
+    // cutoff <= 0, which admits nothing: the walk's first step already leaves the band)
+    for (int t = 0; t < n; ++t) a.env_hi[t] = -1;
+    for (int t = n - 1; t >= 0; --t) {
+        int m = 0;
+        while (m <= n && hi[m] < t + 1) ++m;
+        a.env_lo[t] = (int8_t)(m - 1);
+        if (m >= 1 && m <= n) a.env_hi[m - 1] = (int8_t)t;  // the smallest such t is written last
+    }
+    int d = 0;  // the first sample with a lower bound
+    while (d < n && a.env_lo[d] < 0) ++d;
+    a.ns = n - d;
     Workspace ws{(char*)workspace, workspace_bytes};
-    int* tables = ws.take<int>(2 * (n + 1));
     float* sorted = ws.take<float>((size_t)n * rows * cols);
-    std::vector<int> host(2 * (n + 1));
-    std::copy(lo.begin(), lo.end(), host.begin());
-    std::copy(hi.begin(), hi.end(), host.begin() + (n + 1));
-    // pageable source: cudaMemcpyAsync stages it before returning
-    DPL_CUDA_TRY(cudaMemcpyAsync(tables, host.data(), host.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    if (hi[0] < 0) {
+        DPL_CUDA_TRY(cudaMemsetAsync(is_shp, 0, (size_t)out_rows * out_cols * wy * wx, s));
+        return DPL_OK;
+    }
     const int64_t npix = rows * cols;
     const float* src = amp_stack;
     if (!is_sorted) {
@@ -491,10 +620,7 @@ extern "C" dpl_status dpl_shp_ks(const float* amp_stack, int64_t nslc, int64_t r
         DPL_CUDA_TRY(cudaGetLastError());
         src = sorted;
     }
-    KsArgs a{};
     a.sorted = src;
-    a.lo = tables;
-    a.hi = tables + (n + 1);
     a.n = n;
     a.rows = (int)rows;
     a.cols = (int)cols;
@@ -505,20 +631,21 @@ extern "C" dpl_status dpl_shp_ks(const float* amp_stack, int64_t nslc, int64_t r
     a.out_rows = out_rows;
     a.out_cols = out_cols;
     a.is_shp = is_shp;
-    int tr = 8, tc = 16;
+    // the largest tile of up to 8 x 32 pixels whose samples and mask bits leave room for
+    // two CTAs per SM; windows too large for that get what one CTA can hold
+    int tr = 8, tc = 32;
+    auto region = [&](int r, int c) { return ((size_t)(r - 1) * sy + wy) * ((size_t)(c - 1) * sx + wx); };
     auto smem_for = [&](int r, int c) {
-        size_t rh = (size_t)(r - 1) * sy + wy, rw = (size_t)(c - 1) * sx + wx;
-        return 2 * (n + 1) * sizeof(int) + rh * rw * n * sizeof(float);
+        return region(r, c) * (n | 1) * sizeof(float) + (size_t)r * c * wy * ((wx + 31) / 32) * sizeof(uint32_t);
     };
-    while (smem_for(tr, tc) > 96 * 1024 && (tr > 1 || tc > 1)) {
-        if (tc >= tr && tc > 1) tc /= 2;
+    while (smem_for(tr, tc) > 110 * 1024 && (tr > 1 || tc > 1)) {
+        if (tr * sy >= tc * sx && tr > 1) tr /= 2;
+        else if (tc > 1) tc /= 2;
         else tr /= 2;
     }
-    if (smem_for(tr, tc) > 200 * 1024) return fail(DPL_ERR_UNSUPPORTED, "dpl_shp_ks: window too large");
+    if (smem_for(tr, tc) > 227 * 1024) return fail(DPL_ERR_UNSUPPORTED, "dpl_shp_ks: window too large");
     a.tile_r = tr;
     a.tile_c = tc;
-    size_t smem = smem_for(tr, tc);
-    DPL_CUDA_TRY(cudaFuncSetAttribute(k_ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_ks<<<dim3(ceil_div(out_cols, tc), ceil_div(out_rows, tr)), 256, smem, s>>>(a);
-    return check_launch("k_ks");
+    a.off_bits = (int)region(tr, tc) * (n | 1);
+    return launch_ks<4>(a, dim3(ceil_div(out_cols, tc), ceil_div(out_rows, tr)), smem_for(tr, tc), s);
 }

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "../../include/dpl.h"
+#include "dpl_common.cuh"
 
 namespace dpl {
 
@@ -13,16 +14,19 @@ struct GlrtArgs {
     float thr;
     int tile_r, tile_c;  // output pixels per CTA
     int box_w, box_h;    // TMA box (floats x rows)
-    uint8_t* is_shp;     // (out_rows, out_cols, wy, wx) bytes, or
-    uint32_t* bits;      // (out_rows, out_cols, wy, words_per_row) packed masks
-    int words_per_row;   // 1 (wx <= 32) or 2 (wx <= 64)
+    uint8_t* is_shp;     // (out_rows, out_cols, wy, wx) bytes
+    int ratio;           // the ratio test applies (else logarithms)
+    float four_c;        // 4 exp(thr / nslc)
+    float ratio_max;     // largest scale^2 of the ratio test
     int* status;         // set to DPL_ERR_TIMEOUT if a bounded wait gives up
 };
 
 struct KsArgs {
     const float* sorted;  // (n, rows, cols)
-    const int* lo;
-    const int* hi;
+    int8_t lo[kMaxNslc + 1], hi[kMaxNslc + 1];  // admissible i2 per i1 of the merge walk
+    int8_t env_lo[kMaxNslc], env_hi[kMaxNslc];  // envelope of sample t: indices into x1 (-1: none)
+    int ns;               // samples with a lower bound (n minus the first index that has one)
+    int off_bits;         // the mask bits, in 4-byte words from the start of shared memory
     int n, rows, cols, hy, hx, sy, sx, out_rows, out_cols;
     int tile_r, tile_c;
     uint8_t* is_shp;
@@ -32,9 +36,9 @@ int64_t glrt_pitch(int64_t cols);
 size_t glrt_workspace_size(int64_t rows, int64_t cols);
 size_t ks_workspace_size(int64_t nslc, int64_t rows, int64_t cols);
 
-// scale2: rows x glrt_pitch(cols) floats.  Exactly one of is_shp / bits is non-null.
+// scale2: rows x glrt_pitch(cols) floats.
 dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_t cols, int hy, int hx, int sy,
-                       int sx, int nslc, float threshold, uint8_t* is_shp, uint32_t* bits, int* status,
-                       float* scale2, cudaStream_t s);
+                       int sx, int nslc, float threshold, uint8_t* is_shp, int* status, float* scale2,
+                       cudaStream_t s);
 
 }  // namespace dpl
