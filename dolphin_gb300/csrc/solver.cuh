@@ -264,13 +264,17 @@ __device__ void s_lu_solve(const cfloat* A, int n, const int* src, cfloat (&x)[N
     for (int q = 0; q < NB; ++q) x[q] = w[q];
 }
 
+// |c| by the approximate square root (relative error below 2^-22)
+__device__ __forceinline__ float s_abs_approx(cfloat c) {
+    float g;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(g) : "f"(fmaf(c.re, c.re, c.im * c.im)));
+    return g;
+}
+
 __device__ __forceinline__ float s_gamma(const PixArgs& a, cfloat c, bool diag) {
     // |c|: the correctly rounded square root where the zero-correlation threshold
-    // compares it, the approximate one (relative error below 2^-22) otherwise
-    const float m2 = c.re * c.re + c.im * c.im;
-    float g;
-    if (a.zct > 0.f) g = sqrtf(m2);
-    else asm("sqrt.approx.f32 %0, %1;" : "=f"(g) : "f"(m2));
+    // compares it, the approximate one otherwise
+    float g = a.zct > 0.f ? sqrtf(fmaf(c.re, c.re, c.im * c.im)) : s_abs_approx(c);
     if (a.beta_on) g = fadd(fmul(a.one_minus_beta, g), diag ? a.beta : 0.f);
     return g < a.zct ? 0.f : g;
 }

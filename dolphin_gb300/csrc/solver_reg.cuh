@@ -15,40 +15,60 @@
 //        listed for the LU pass (the reference's LU algorithm), as in solve_pixel.
 //   EVD: power iteration on C o |C| with the rows in registers (_eigenvalues.py:93-136).
 //
-// Register rotation keeps the sweeps in compact loops: before step k, slot s of a
-// row holds column (k + s) mod K, so the pivot column is always slot 0 and each
-// update writes slot s - 1 from slot s (the shift costs nothing).  The column is
-// broadcast through shared memory at position (row - k) mod K, so slot s reads
-// position s.  Rows and columns >= N are zero and stay zero.
+// What bounds it: no single pipe, but issue slots, the shared-memory reads of the
+// broadcast columns (a 16-byte broadcast costs the SM about two cycles) and instruction
+// fetch: code that a pixel runs once, unrolled, costs several times more cycles per
+// instruction than the sweep loops, so options that few runs use (baseline lag, beta,
+// zero-correlation threshold, zero entries in the temporal coherence) sit in rolled loops
+// apart, and divergent stores are selects.
+//
+// Packed arithmetic: a row's K values are held as K / 2 pairs of neighbouring columns
+// (complex rows as a real and an imaginary plane), and the sweeps, the matrix-vector
+// product and the element-wise builds use two-wide multiply-adds (one issue slot for two
+// IEEE operations).  Every element sees the operations of the scalar form in the same
+// order: phases, CRLB and estimator are the same bit for bit.  One pixel-warp at K = 30,
+// alone on the SM: a real sweep 2594 -> 2041 cycles, the Hermitian one 6982 -> 5268.
+//
+// 1034 x 1046 pixels at N = 30: 17.3 -> 14.2 ms.
+//
+// Register rotation keeps the sweeps in compact loops: before the steps k, k + 1 (k
+// even), slot s of a row holds column (k + s) mod K, so the pivot columns are slots 0 and
+// 1.  Step k updates in place; step k + 1 writes pair q - 1 from pair q (the shift by one
+// pair costs nothing).  Both columns are broadcast through shared memory at position
+// (row - k) mod K, so slot s reads position s.  Rows and columns N .. K - 1 are padded
+// with the identity, whose steps change nothing.
 #pragma once
 
 namespace dpl {
 
-// Shared memory per pixel group: full Hermitian C (n x ld, ld odd: a thread-per-row
-// access of one column is conflict-free), |Gamma| / |Gamma|^{-1} (n x ld floats), a
-// 128-entry broadcast buffer, a 64-entry vector buffer and reduction slots.
-struct RegLayout {
-    int ld;
-    size_t off_C, off_G, off_b, off_w, off_x, bytes;
-};
-
-inline RegLayout make_reg_layout(int n) {
-    RegLayout L{};
-    L.ld = n | 1;
-    size_t o = 0;
-    auto take = [&](size_t bytes) {
-        size_t at = o;
-        o = align_up(o + bytes, 16);
-        return at;
-    };
-    L.off_C = take((size_t)n * L.ld * sizeof(cfloat));
-    L.off_G = take((size_t)n * L.ld * sizeof(float));
-    L.off_b = take(128 * sizeof(cfloat));  // the sweeps' two broadcast halves
-    L.off_w = take(64 * sizeof(cfloat));
-    L.off_x = take(16 * sizeof(float));
-    L.bytes = align_up(o, 128);
-    return L;
+// two floats in one 64-bit register pair, with two IEEE operations per instruction
+typedef float2 f2;
+__device__ __forceinline__ f2 f2_pack(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ float f2_lo(f2 v) { return v.x; }
+__device__ __forceinline__ float f2_hi(f2 v) { return v.y; }
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ f2 f2_ld(const float* p, int q) { return reinterpret_cast<const float2*>(p)[q]; }
+__device__ __forceinline__ void f2_ld2(const float* p, int q, f2& a, f2& b) {  // pairs 2q, 2q + 1
+    const float4 t = reinterpret_cast<const float4*>(p)[q];
+    a = f2_pack(t.x, t.y);
+    b = f2_pack(t.z, t.w);
 }
+__device__ __forceinline__ void f2_st(float* p, int q, f2 v) { reinterpret_cast<float2*>(p)[q] = v; }
+
+// Shared memory of a pixel group: three K x LD planes (Re and Im of the full Hermitian C,
+// and |Gamma| or its inverse), a buffer for the broadcast columns (two halves of two
+// planes) and vectors, and (two-warp groups) reduction slots.  LD is even with LD / 2
+// odd: a thread per row reading pairs is conflict-free.
+template <int K, int G>
+struct RegShape {
+    static constexpr int LD = (K / 2) % 2 ? K : K + 2;
+    static constexpr int KB = (K + 3) & ~3;  // a plane of a broadcast column or vector
+    static constexpr int NP = (K * (K - 1) / 2 + G - 1) / G;  // lower pairs per thread
+    static constexpr int PLANE = K * LD;
+    static constexpr int OFF_U = 3 * PLANE, OFF_X = OFF_U + 4 * KB;
+    static constexpr int FLOATS = (OFF_X + (G == 64 ? 16 : 0) + 31) & ~31;
+};
 
 // A pixel group of G threads: G = 8, 16 or 32 lanes of one warp (a warp holds 32 / G
 // pixels) or G = 64, two whole warps: row index, synchronisation, reductions.
@@ -116,132 +136,238 @@ __device__ __forceinline__ float frcp_nr(float p) {
 
 // The sweeps broadcast the pivot column through `buf`, two halves used alternately so
 // that one barrier per step suffices: step k writes half k & 1, whose readers (step
-// k - 2) all passed step k - 1's barrier before this thread did.  Row `gl` writes its
-// pivot-column entry at position (gl - k) mod K, so slot s of every row reads position s.
+// k - 2) all passed step k - 1's barrier before this thread did.
 
-// Real symmetric sweep over indices 0..n-1 of the matrix whose row `gl` is g; on
-// success g holds row `gl` of -A^{-1}.  Returns false (uniformly) if any pivot was
-// <= 0 (the remaining steps then run on meaningless values, without branching).
-// buf: 2 * ((K + 3) & ~3) floats.
+// Real symmetric sweep of the matrix whose row `gl` is g; on success g holds row `gl` of
+// -A^{-1}.  Returns false (uniformly) if any pivot was <= 0 (the remaining steps then run
+// on meaningless values, without branching).  buf: 2 * KB floats.
 template <int K, int G>
-__device__ __forceinline__ bool r_sweep(float (&g)[K], int n, float* buf, const Grp<G>& gr) {
-    constexpr int KB = (K + 3) & ~3;  // half stride: 16-byte aligned
-    bool bad = false;                 // uniform: every thread reads the same pivot
+__device__ __forceinline__ bool r_sweep(f2 (&g)[K / 2], float* buf, const Grp<G>& gr) {
+    constexpr int KB = RegShape<K, G>::KB;
+    bool bad = false;  // uniform: every thread reads the same pivot
     int pos = gr.gl;
     gr.sync();  // earlier users of buf are done with it
 #pragma unroll 1
-    for (int k = 0; k < n; ++k) {
-        float* bk = buf + (k & 1) * KB;
-        if (gr.gl < K) bk[pos] = g[0];  // A[row][k] (= A[k][row])
-        gr.sync();
-        float r[K];
-        const float4* b4 = reinterpret_cast<const float4*>(bk);
+    for (int k = 0; k < K; k += 2) {
+        {
+            const float g0 = f2_lo(g[0]);
+            if (gr.gl < K) buf[pos] = g0;  // A[row][k] (= A[k][row])
+            gr.sync();
+            const float p = buf[0];
+            bad |= !(p > 0.f);
+            const float ip = frcp_nr(p);
+            const bool me = gr.gl == k;
+            // rows i != k: a_ij - (a_ik / p) a_kj; row k: a_kj / p, written as
+            // a_kj - (1 - 1/p) a_kj so that every thread runs the same FMA
+            const float t = me ? 1.f - ip : g0 * ip;
+            const float last = me ? -ip : g0 * ip;
+            const f2 nt = f2_pack(-t, -t);
 #pragma unroll
-        for (int q = 0; q < K / 4; ++q) {
-            const float4 t = b4[q];
-            r[4 * q] = t.x;
-            r[4 * q + 1] = t.y;
-            r[4 * q + 2] = t.z;
-            r[4 * q + 3] = t.w;
+            for (int q = 0; q < K / 4; ++q) {
+                f2 x, y;
+                f2_ld2(buf, q, x, y);
+                g[2 * q] = f2_fma(nt, x, g[2 * q]);
+                g[2 * q + 1] = f2_fma(nt, y, g[2 * q + 1]);
+            }
+            if (K % 4) g[K / 2 - 1] = f2_fma(nt, f2_ld(buf, K / 2 - 1), g[K / 2 - 1]);
+            g[0] = f2_pack(last, f2_hi(g[0]));
         }
-        if (K % 4) {  // K = 4m + 2: the last two slots
-            const float2 t = reinterpret_cast<const float2*>(bk)[K / 2 - 1];
-            r[K - 2] = t.x;
-            r[K - 1] = t.y;
+        {
+            const float g1 = f2_hi(g[0]);
+            float* b1 = buf + KB;
+            if (gr.gl < K) b1[pos] = g1;
+            gr.sync();
+            const float p = b1[1];
+            bad |= !(p > 0.f);
+            const float ip = frcp_nr(p);
+            const bool me = gr.gl == k + 1;
+            const float t = me ? 1.f - ip : g1 * ip;
+            const float last = me ? -ip : g1 * ip;
+            const f2 nt = f2_pack(-t, -t);
+            f2 first = f2_pack(0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < K / 4; ++q) {
+                f2 x, y;
+                f2_ld2(b1, q, x, y);
+                if (q == 0) first = f2_fma(nt, x, g[0]);
+                else g[2 * q - 1] = f2_fma(nt, x, g[2 * q]);
+                g[2 * q] = f2_fma(nt, y, g[2 * q + 1]);
+            }
+            if (K % 4) g[K / 2 - 2] = f2_fma(nt, f2_ld(b1, K / 2 - 1), g[K / 2 - 1]);
+            g[K / 2 - 1] = f2_pack(f2_lo(first), last);
         }
-        const float p = r[0];
-        bad |= !(p > 0.f);
-        const float ip = frcp_nr(p);
-        const bool me = gr.gl == k;
-        // rows i != k: a_ij - (a_ik / p) a_kj; row k: a_kj / p, written as
-        // a_kj - (1 - 1/p) a_kj so that every thread runs the same FMA
-        const float t = me ? 1.f - ip : g[0] * ip;
-        const float last = me ? -ip : g[0] * ip;
-#pragma unroll
-        for (int s = 0; s < K - 1; ++s) g[s] = fmaf(-t, r[s + 1], g[s + 1]);
-        g[K - 1] = last;
-        pos = pos == 0 ? K - 1 : pos - 1;
-    }
-#pragma unroll 1
-    for (int k = n; k < K; ++k) {  // finish the rotation: slot s holds column s again
-        const float t0 = g[0];
-#pragma unroll
-        for (int s = 0; s < K - 1; ++s) g[s] = g[s + 1];
-        g[K - 1] = t0;
+        pos -= 2;
+        pos = pos < 0 ? pos + K : pos;
     }
     gr.sync();
     return !bad;
 }
 
-// Hermitian sweep: on success a holds row `gl` of -A^{-1}.  False if a pivot was <= 0.
-// buf: 2 * K complex.
+// Hermitian sweep: on success (re, im) hold row `gl` of -A^{-1}.  False if a pivot was
+// <= 0.  buf: 4 * KB floats.
 template <int K, int G>
-__device__ __forceinline__ bool r_sweep_c(cfloat (&a)[K], int n, cfloat* buf, const Grp<G>& gr) {
+__device__ __forceinline__ bool r_sweep_c(f2 (&re)[K / 2], f2 (&im)[K / 2], float* buf, const Grp<G>& gr) {
+    constexpr int KB = RegShape<K, G>::KB;
     bool bad = false;  // uniform: every thread reads the same pivot
     int pos = gr.gl;
     gr.sync();
 #pragma unroll 1
-    for (int k = 0; k < n; ++k) {
-        cfloat* bk = buf + (k & 1) * K;  // K even: 16-byte aligned halves
-        if (gr.gl < K) bk[pos] = a[0];   // A[row][k] = conj(A[k][row])
-        gr.sync();
-        const float p = bk[0].re;
-        bad |= !(p > 0.f);
-        const float ip = frcp_nr(p);
-        const bool me = gr.gl == k;
-        const cfloat t = me ? cmake(1.f - ip, 0.f) : cscale(a[0], ip);
-        const cfloat last = me ? cmake(-ip, 0.f) : cscale(a[0], ip);
-        const float4* b4 = reinterpret_cast<const float4*>(bk);
-#pragma unroll
-        for (int q = 0; q < K / 2; ++q) {
-            const float4 b = b4[q];
+    for (int k = 0; k < K; k += 2) {
+        {
+            const float a0 = f2_lo(re[0]), c0 = f2_lo(im[0]);
+            if (gr.gl < K) {  // A[row][k] = conj(A[k][row])
+                buf[pos] = a0;
+                buf[KB + pos] = c0;
+            }
+            gr.sync();
+            const float p = buf[0];
+            bad |= !(p > 0.f);
+            const float ip = frcp_nr(p);
+            const bool me = gr.gl == k;
+            const float sr = a0 * ip, si = c0 * ip;
+            const float tr = me ? 1.f - ip : sr, ti = me ? 0.f : si;
+            const f2 ntr = f2_pack(-tr, -tr), nti = f2_pack(-ti, -ti), ptr = f2_pack(tr, tr);
             // slot s: a_ij - t a_kj, a_kj = conj(buffer entry s)
-            if (q > 0) a[2 * q - 1] = cfms_conj(a[2 * q], t, cmake(b.x, b.y));
-            a[2 * q] = cfms_conj(a[2 * q + 1], t, cmake(b.z, b.w));
-        }
-        a[K - 1] = last;
-        pos = pos == 0 ? K - 1 : pos - 1;
-    }
-#pragma unroll 1
-    for (int k = n; k < K; ++k) {
-        const cfloat t0 = a[0];
+            auto update = [&](int q, f2 br, f2 bi) {
+                re[q] = f2_fma(ntr, br, f2_fma(nti, bi, re[q]));
+                im[q] = f2_fma(nti, br, f2_fma(ptr, bi, im[q]));
+            };
 #pragma unroll
-        for (int s = 0; s < K - 1; ++s) a[s] = a[s + 1];
-        a[K - 1] = t0;
+            for (int q = 0; q < K / 4; ++q) {
+                f2 r0, r1, i0, i1;
+                f2_ld2(buf, q, r0, r1);
+                f2_ld2(buf + KB, q, i0, i1);
+                update(2 * q, r0, i0);
+                update(2 * q + 1, r1, i1);
+            }
+            if (K % 4) update(K / 2 - 1, f2_ld(buf, K / 2 - 1), f2_ld(buf + KB, K / 2 - 1));
+            re[0] = f2_pack(me ? -ip : sr, f2_hi(re[0]));
+            im[0] = f2_pack(me ? 0.f : si, f2_hi(im[0]));
+        }
+        {
+            float* b1 = buf + 2 * KB;
+            const float a1 = f2_hi(re[0]), c1 = f2_hi(im[0]);
+            if (gr.gl < K) {
+                b1[pos] = a1;
+                b1[KB + pos] = c1;
+            }
+            gr.sync();
+            const float p = b1[1];
+            bad |= !(p > 0.f);
+            const float ip = frcp_nr(p);
+            const bool me = gr.gl == k + 1;
+            const float sr = a1 * ip, si = c1 * ip;
+            const float tr = me ? 1.f - ip : sr, ti = me ? 0.f : si;
+            const f2 ntr = f2_pack(-tr, -tr), nti = f2_pack(-ti, -ti), ptr = f2_pack(tr, tr);
+            f2 fr = f2_pack(0.f, 0.f), fi = f2_pack(0.f, 0.f);
+            auto update = [&](int q, f2 br, f2 bi) {  // pair q into pair q - 1
+                const f2 x = f2_fma(ntr, br, f2_fma(nti, bi, re[q]));
+                const f2 y = f2_fma(nti, br, f2_fma(ptr, bi, im[q]));
+                if (q == 0) {
+                    fr = x;
+                    fi = y;
+                } else {
+                    re[q - 1] = x;
+                    im[q - 1] = y;
+                }
+            };
+#pragma unroll
+            for (int q = 0; q < K / 4; ++q) {
+                f2 r0, r1, i0, i1;
+                f2_ld2(b1, q, r0, r1);
+                f2_ld2(b1 + KB, q, i0, i1);
+                update(2 * q, r0, i0);
+                update(2 * q + 1, r1, i1);
+            }
+            if (K % 4) update(K / 2 - 1, f2_ld(b1, K / 2 - 1), f2_ld(b1 + KB, K / 2 - 1));
+            re[K / 2 - 1] = f2_pack(f2_lo(fr), me ? -ip : sr);
+            im[K / 2 - 1] = f2_pack(f2_lo(fi), me ? 0.f : si);
+        }
+        pos -= 2;
+        pos = pos < 0 ? pos + K : pos;
     }
     gr.sync();
     return !bad;
 }
 
-// y_row = sum_j h[j] x_j (row `gl` of a matrix in registers); x published in vb
+// Publishes a vector as three planes (Re, Im, -Im) of KB floats.
 template <int K, int G>
-__device__ __forceinline__ cfloat r_matvec(const cfloat (&h)[K], cfloat x, cfloat* vb, const Grp<G>& gr) {
+__device__ __forceinline__ void r_publish(float* vb, cfloat x, const Grp<G>& gr) {
+    constexpr int KB = RegShape<K, G>::KB;
     gr.sync();
-    vb[gr.gl] = x;
-    gr.sync();
-    const float4* v4 = reinterpret_cast<const float4*>(vb);
-    cfloat acc0 = cmake(0.f, 0.f), acc1 = cmake(0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < K / 2; ++q) {
-        const float4 t = v4[q];
-        acc0 = cfma(acc0, h[2 * q], cmake(t.x, t.y));
-        acc1 = cfma(acc1, h[2 * q + 1], cmake(t.z, t.w));
+    if (gr.gl < K) {
+        vb[gr.gl] = x.re;
+        vb[KB + gr.gl] = x.im;
+        vb[2 * KB + gr.gl] = -x.im;
     }
-    return cadd(acc0, acc1);
+    gr.sync();
 }
 
-// Asynchronous copy of one pixel's planar coherence (count floats) into shared memory.
-template <int G>
-__device__ __forceinline__ void r_prefetch(float* dst, const float* src, int count, const Grp<G>& gr) {
-    gr.sync();
-    // 4-byte pieces: 16-byte copies measured slower here (the solve is issue-bound and
-    // the copy has the whole temporal-coherence pass to land)
-    for (int e = gr.gl; e < count; e += G)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + e)),
-                     "l"(src + e)
-                     : "memory");
-    asm volatile("cp.async.commit_group;" ::: "memory");
+// y_row = sum_j h_j x_j (row `gl` of a matrix in registers), even and odd columns summed
+// apart; x published in vb
+template <int K, int G>
+__device__ __forceinline__ cfloat r_matvec(const f2 (&hr)[K / 2], const f2 (&hi)[K / 2], cfloat x, float* vb,
+                                           const Grp<G>& gr) {
+    constexpr int KB = RegShape<K, G>::KB;
+    r_publish<K, G>(vb, x, gr);
+    f2 ar = f2_pack(0.f, 0.f), ai = f2_pack(0.f, 0.f);
+    auto step = [&](int q, f2 r, f2 i, f2 n) {
+        ar = f2_fma(hr[q], r, f2_fma(hi[q], n, ar));
+        ai = f2_fma(hr[q], i, f2_fma(hi[q], r, ai));
+    };
+#pragma unroll
+    for (int q = 0; q < K / 4; ++q) {
+        f2 r0, r1, i0, i1, n0, n1;
+        f2_ld2(vb, q, r0, r1);
+        f2_ld2(vb + KB, q, i0, i1);
+        f2_ld2(vb + 2 * KB, q, n0, n1);
+        step(2 * q, r0, i0, n0);
+        step(2 * q + 1, r1, i1, n1);
+    }
+    if (K % 4) step(K / 2 - 1, f2_ld(vb, K / 2 - 1), f2_ld(vb + KB, K / 2 - 1), f2_ld(vb + 2 * KB, K / 2 - 1));
+    if (gr.gl >= K) return cmake(0.f, 0.f);  // lanes beyond the matrix
+    return cmake(f2_lo(ar) + f2_hi(ar), f2_lo(ai) + f2_hi(ai));
 }
+
+// One pixel's input in registers: the diagonal entry of row `gl` and the lower pairs
+// e = gl, gl + G, ... (planar sums, or entries of a full matrix).  Fetched for the next
+// pixel while the current one's temporal coherence runs, when the matrix rows are dead.
+template <int K, int G>
+struct RegFetch {
+    float2 v[RegShape<K, G>::NP];
+    float2 d;
+    __device__ __forceinline__ void load(const PixArgs& a, int64_t p, const uint16_t* ptab, int gl) {
+        const int n = a.n, npairs = n * (n - 1) / 2;
+        d = make_float2(0.f, 0.f);
+        if (a.Cplanar) {
+            const float* src = a.Cplanar + p * n * n;
+            if (gl < n) d.x = src[gl];
+            src += n;
+            if (n & 1) {  // the pairs lie on 4-byte boundaries in every other pixel
+#pragma unroll
+                for (int i = 0; i < RegShape<K, G>::NP; ++i) {
+                    const int e = gl + i * G;
+                    v[i] = e < npairs ? make_float2(src[2 * e], src[2 * e + 1]) : make_float2(0.f, 0.f);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < RegShape<K, G>::NP; ++i) {
+                    const int e = gl + i * G;
+                    v[i] = e < npairs ? reinterpret_cast<const float2*>(src)[e] : make_float2(0.f, 0.f);
+                }
+            }
+        } else {
+            const float2* src = reinterpret_cast<const float2*>(a.Cin) + p * n * n;
+            if (gl < n) d = src[gl * n + gl];
+#pragma unroll
+            for (int i = 0; i < RegShape<K, G>::NP; ++i) {
+                const int e = gl + i * G;
+                const uint32_t rc = e < npairs ? ptab[e] : 0u;
+                v[i] = src[(rc & 0xff) * n + (rc >> 8)];
+            }
+        }
+    }
+};
 
 // Normalising iteration x <- op(v) / |op(v)| until |x - v| <= 1e-5 or 49 steps
 // (the reference's while-loop: iteration count starts at 1, stops below 50).  Adds the
@@ -260,122 +386,150 @@ __device__ __forceinline__ float r_iterate(cfloat& v, const Grp<G>& gr, int& ste
     return diff;
 }
 
-// Full solve for one pixel whose Hermitian coherence matrix is in Cf (n x ld, both
-// triangles).  A pixel whose shifted EMI matrix is not positive definite is appended
-// to a.fb_list and left for the LU pass.  Once Gs is no longer needed, the planar
-// coherence of the group's next pixel (`next`, if any) is prefetched into it.
-template <int K, int G>
-__device__ void solve_pixel_reg(const PixArgs& a, int64_t p, const cfloat* Cf, float* Gs, int ld, cfloat* cb,
-                                cfloat* wb, const uint32_t* ptab, const float* next, const Grp<G>& gr) {
+// Full solve for one pixel whose Hermitian coherence matrix is in the planes Cr, Ci (both
+// triangles) and whose |Gamma| is in Gs off the diagonal.  A pixel whose shifted EMI
+// matrix is not positive definite is appended to a.fb_list and left for the LU pass.
+// `fetch` loads the group's next pixel.
+template <int K, int G, class Fetch>
+__device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, float* Cr, float* Ci, float* Gs, float* U,
+                                                const uint16_t* ptab, const Grp<G>& gr, Fetch&& fetch) {
+    using S = RegShape<K, G>;
+    constexpr int LD = S::LD, KB = S::KB;
     const int n = a.n, me = gr.gl;
-    const bool row = me < n;
-    const cfloat* Ci = Cf + (row ? me : 0) * ld;
+    const bool row = me < n, act = me < K;  // a row of the matrix; a row of the padded one
+    const int mrow = act ? me : 0;
+    float* cr = Cr + mrow * LD;
+    float* ci = Ci + mrow * LD;
+    float* Gi = Gs + mrow * LD;
     if (a.closure && me < n - 2) {
-        const cfloat c = cmulc(cmul(Cf[me * ld + me + 1], Cf[(me + 1) * ld + me + 2]), Cf[me * ld + me + 2]);
+        const cfloat c01 = cmake(Cr[me * LD + me + 1], Ci[me * LD + me + 1]);
+        const cfloat c12 = cmake(Cr[(me + 1) * LD + me + 2], Ci[(me + 1) * LD + me + 2]);
+        const cfloat c02 = cmake(Cr[me * LD + me + 2], Ci[me * LD + me + 2]);
+        const cfloat c = cmulc(cmul(c01, c12), c02);
         a.closure[p * (n - 2) + me] = atan2f(c.im, c.re);
     }
-    // |Gamma| + 1e-6 I -> -|Gamma|^{-1} (round 0), then the CRLB's Fisher matrix
-    // FIM = 2L (Gamma o Gamma^{-1} - I), row/col `ref` -> identity, + 1e-6 I (round 1).
-    // Gs holds |Gamma| during round 0 and |Gamma|^{-1} afterwards.
-    float* Gi = Gs + (row ? me : 0) * ld;
     const int ref = a.crlb_ref;
     bool inv_nan = true;
     bool crlb_ok = false;
     float dg = 0.f;
     if (!(a.use_evd && !a.compute_crlb)) {
-        // |Gamma| + 1e-6 I into shared memory by lower pairs (every thread busy), the
-        // diagonal of |Gamma| itself kept in gdiag, then into the register slots
-        const int nr = row ? n : 0;  // this row's live columns
-        const int npairs = n * (n - 1) / 2;
-        for (int e = me; e < npairs; e += G) {
-            const uint32_t rc = ptab[e];
-            const int r = rc & 0xffff, c = rc >> 16;
-            const float gm = s_gamma(a, Cf[r * ld + c], false);
-            Gs[r * ld + c] = gm;
-            Gs[c * ld + r] = gm;
-        }
+        // |Gamma| + 1e-6 I -> -|Gamma|^{-1} (round 0), then the CRLB's Fisher matrix
+        // FIM = 2L (Gamma o Gamma^{-1} - I), row/col `ref` -> identity, + 1e-6 I (round 1).
+        // Gs holds |Gamma| during round 0 and |Gamma|^{-1} afterwards.
         float gdiag = 0.f;
         if (row) {
-            gdiag = s_gamma(a, Ci[me], true);
+            gdiag = s_gamma(a, cmake(cr[me], ci[me]), true);
             Gi[me] = fadd(gdiag, 1e-6f);
+        } else if (act) {
+            Gi[me] = 1.f;
         }
-        gr.sync();
-        float g[K];
+        f2 g[K / 2];
 #pragma unroll
-        for (int j = 0; j < K; ++j) g[j] = j < nr ? Gi[j] : 0.f;
+        for (int q = 0; q < K / 2; ++q) g[q] = f2_ld(Gi, q);
 #pragma unroll 1
         for (int round = 0; round < 2; ++round) {
-            const bool ok = r_sweep<K, G>(g, n, reinterpret_cast<float*>(cb), gr);
+            const bool ok = r_sweep<K, G>(g, U, gr);
             if (round == 1) {
                 crlb_ok = ok;
 #pragma unroll
-                for (int j = 0; j < K; ++j)
-                    if (j == me) dg = g[j];
+                for (int q = 0; q < K / 2; ++q) {
+                    if (me == 2 * q) dg = f2_lo(g[q]);
+                    if (me == 2 * q + 1) dg = f2_hi(g[q]);
+                }
                 break;
             }
             inv_nan = !ok;
             if (ok) {
-                bool bad = false;
+                f2 z = f2_pack(0.f, 0.f);  // NaN if any entry is NaN or infinite
 #pragma unroll
-                for (int j = 0; j < K; ++j) bad |= isnan(g[j]);
-                inv_nan = gr.any(bad);
-            }
-            // keep |Gamma|^{-1} and build the FIM in place of it
-            const bool refrow = me == ref;
+                for (int q = 0; q < K / 2; ++q) z = f2_fma(g[q], f2_pack(0.f, 0.f), z);
+                const float zs = f2_lo(z) + f2_hi(z);
+                if (gr.any(row && isnan(zs))) {
+                    bool nan = false;
 #pragma unroll
-            for (int j = 0; j < K; ++j) {
-                const float ginv = -g[j];
-                float x = 0.f;
-                if (j < nr) {
-                    const bool dj = j == me;
-                    x = fmul(a.crlb_factor, fsub(fmul(dj ? gdiag : Gi[j], ginv), dj ? 1.f : 0.f));
-                    if (dj) x = fadd(x, 1e-6f);
-                    if (refrow || j == ref) x = dj ? 1.f : 0.f;
-                    Gi[j] = ginv;
+                    for (int q = 0; q < K / 2; ++q) nan |= isnan(f2_lo(g[q])) || isnan(f2_hi(g[q]));
+                    inv_nan = gr.any(row && nan);
                 }
-                g[j] = x;
             }
-            if (!a.compute_crlb || inv_nan) break;
+            if (inv_nan) break;  // Gs keeps its finite padding
+            // keep |Gamma|^{-1} and build the FIM in place of it; the identity rows (the
+            // reference's, the padding) are 0 with 1 on the diagonal
+            const bool unit = me == ref || !row;
+            const float f = unit ? 0.f : a.crlb_factor;
+            const float dsub = unit ? 0.f : 1.f, dadd = unit ? 1.f : 1e-6f;
+            if (row) {
+                Gi[me] = gdiag;
+                if (a.compute_crlb) Gi[ref] = 0.f;
+            }
+            const f2 ff = f2_pack(f, f), minus = f2_pack(-1.f, -1.f);
+#pragma unroll
+            for (int q = 0; q < K / 2; ++q) {
+                const f2 ginv = f2_mul(g[q], minus);
+                const f2 gm = f2_ld(Gi, q);
+                if (act) f2_st(Gi, q, ginv);
+                const f2 y = f2_mul(gm, ginv);
+                float y0 = f2_lo(y), y1 = f2_hi(y);
+                if (me == 2 * q) y0 = fsub(y0, dsub);
+                if (me == 2 * q + 1) y1 = fsub(y1, dsub);
+                const f2 x = f2_mul(ff, f2_pack(y0, y1));
+                float x0 = f2_lo(x), x1 = f2_hi(x);
+                if (me == 2 * q) x0 = fadd(x0, dadd);
+                if (me == 2 * q + 1) x1 = fadd(x1, dadd);
+                g[q] = f2_pack(x0, x1);
+            }
+            if (!a.compute_crlb) break;
         }
     }
     const bool evd = a.use_evd || inv_nan;
     if (row) a.crlb[p * n + me] = !a.compute_crlb || me == ref ? 0.f : (crlb_ok ? sqrtf(-dg) : nanf(""));
 
+    // One matrix (re, im) and one iteration for both estimators, the matrix formed as
+    // C o Gs: EMI iterates with -(A - 0.99 I)^{-1} (the negated sweep result), its
+    // shifted diagonal put into Gs against a diagonal of 1 in C for the time of the
+    // build; EVD iterates with C o |C|, |C| put into Gs.
+    const int npairs = n * (n - 1) / 2;
+    const float cd = cr[mrow], gd = Gi[mrow];
+    if (!evd) {
+        if (act) {
+            Gi[me] = row ? fsub(cd * gd, 0.99f) : 1.f;
+            cr[me] = 1.f;
+        }
+    } else {
+        gr.sync();
+        for (int e = me; e < npairs; e += G) {
+            const uint32_t rc = ptab[e];
+            const int r = rc & 0xff, c = rc >> 8;
+            const float x = Cr[r * LD + c], y = Ci[r * LD + c];
+            const float m = sqrtf(fmaf(x, x, y * y));
+            Gs[r * LD + c] = m;
+            Gs[c * LD + r] = m;
+        }
+        if (row) Gi[me] = sqrtf(fmaf(cd, cd, ci[me] * ci[me]));
+        gr.sync();
+    }
+    f2 re[K / 2], im[K / 2];
+#pragma unroll
+    for (int q = 0; q < K / 2; ++q) {
+        const f2 gq = f2_ld(Gi, q);
+        re[q] = f2_mul(f2_ld(cr, q), gq);
+        im[q] = f2_mul(f2_ld(ci, q), gq);
+    }
+    if (!evd) {
+        if (act) {
+            Gi[me] = gd;
+            cr[me] = cd;
+        }
+        if (!r_sweep_c<K, G>(re, im, U, gr)) {
+            if (me == 0) a.fb_list[atomicAdd(a.fb_count, 1)] = (int)p;
+            fetch();
+            return;
+        }
+    }
     cfloat v = row ? cmake(1.f / sqrtf((float)n), 0.f) : cmake(0.f, 0.f);
     float lambda;
     int steps = 0;
-    // one matrix slot array and one iteration for both estimators: EMI iterates with
-    // -(A - 0.99 I)^{-1} (the negated sweep result), EVD with C o |C|
-    cfloat mat[K];
-    if (!evd) {
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            cfloat x = cmake(0.f, 0.f);
-            if (row && j < n) {
-                x = cscale(Ci[j], Gi[j]);
-                if (j == me) x.re = fsub(x.re, 0.99f);
-            }
-            mat[j] = x;
-        }
-        if (!r_sweep_c<K, G>(mat, n, cb, gr)) {
-            if (me == 0) a.fb_list[atomicAdd(a.fb_count, 1)] = (int)p;
-            if (next) r_prefetch<G>(Gs, next, n * n, gr);
-            gr.sync();
-            return;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            cfloat x = cmake(0.f, 0.f);
-            if (row && j < n) {
-                const cfloat c = Ci[j];
-                x = cscale(c, sqrtf(c.re * c.re + c.im * c.im));
-            }
-            mat[j] = x;
-        }
-    }
     const float sgn = evd ? 1.f : -1.f;
-    auto op = [&](cfloat x) { return cscale(r_matvec<K, G>(mat, x, wb, gr), sgn); };
+    auto op = [&](cfloat x) { return cscale(r_matvec<K, G>(re, im, x, U, gr), sgn); };
     bool warm = false;
     if (a.vstart && !evd) {
         // learned starting vector; plain EMI (constant start) if it is unusable or the
@@ -397,22 +551,25 @@ __device__ void solve_pixel_reg(const PixArgs& a, int64_t p, const cfloat* Cf, f
     if (diff > 1e-5f && a.nc_list && me == 0) a.nc_list[atomicAdd(a.nc_count, 1)] = (int)p;
     if (!evd) {
         // lambda = Re v^H A v, A_ij = |Gamma|^{-1}_ij C_ij
-        gr.sync();
-        wb[me] = v;
-        gr.sync();
-        cfloat acc = cmake(0.f, 0.f);
-        if (row) {
-            for (int j = 0; j < n; ++j) acc = cfma(acc, cscale(Ci[j], Gi[j]), wb[j]);
+        r_publish<K, G>(U, v, gr);
+        f2 ar = f2_pack(0.f, 0.f), ai = f2_pack(0.f, 0.f);
+#pragma unroll
+        for (int q = 0; q < K / 2; ++q) {
+            const f2 gq = f2_ld(Gi, q);
+            const f2 hr = f2_mul(f2_ld(cr, q), gq), hi = f2_mul(f2_ld(ci, q), gq);
+            const f2 xr = f2_ld(U, q), xi = f2_ld(U + KB, q);
+            ar = f2_fma(hr, xr, f2_fma(hi, f2_ld(U + 2 * KB, q), ar));
+            ai = f2_fma(hr, xi, f2_fma(hi, xr, ai));
         }
-        if (next) r_prefetch<G>(Gs, next, n * n, gr);
+        const cfloat acc = row ? cmake(f2_lo(ar) + f2_hi(ar), f2_lo(ai) + f2_hi(ai)) : cmake(0.f, 0.f);
         const float n2 = gr.sum(cabs2(v));
         lambda = gr.sum(v.re * acc.re + v.im * acc.im);
         v = cscale(v, sqrtf((float)n) / sqrtf(n2));
     } else {
-        if (next) r_prefetch<G>(Gs, next, n * n, gr);
         const cfloat y = op(v);
         lambda = gr.sum(v.re * y.re + v.im * y.im);
     }
+    fetch();  // the matrix rows are dead: the next pixel's values travel during what follows
     // reference to reference_idx
     const cfloat rot = cconj(fphasor(gr.bcast(v, a.ref_idx)));
     v = cmul(v, rot);
@@ -422,45 +579,73 @@ __device__ void solve_pixel_reg(const PixArgs& a, int64_t p, const cfloat* Cf, f
         a.est[p] = evd ? 0 : 1;
         if (a.iters) a.iters[p] = (int16_t)steps;
     }
-    // temporal coherence over pairs c < r (ptab: the lower pairs r | c << 16, row by
-    // row): conj(phasor(C_rc) w_c conj(w_r))
-    gr.sync();
-    wb[me] = fphasor(v);
-    gr.sync();
-    float sre = 0.f, sim = 0.f, cnt = 0.f;
-    const int npairs = n * (n - 1) / 2;
+    // temporal coherence |mean over pairs c < r of conj(phasor(C_rc) w_c conj(w_r))|.
+    // Thread i takes the pairs (i, j), j = i + d mod n, d = 1 .. n / 2: each pair once and
+    // every thread as many.  With x = phasor(C_ij) w_j the pair adds x conj(w_i) where
+    // i < j and its conjugate where i > j: the real part needs the sum of the x, the
+    // imaginary part their sum with the sign of j - i.  A zero or NaN entry makes the sums
+    // NaN: those pixels (and all with a baseline lag, which zeroes entries) take the
+    // pairs one by one and leave NaN pairs out.
+    const cfloat w = fphasor(v);
+    r_publish<K, G>(U, w, gr);
+    float sre = 0.f, sim = 0.f, cnt = (float)npairs;
+    if (row) {
+        float pr = 0.f, pi = 0.f, qr = 0.f, qi = 0.f;
+        const int half = (n - 1) / 2 + ((n & 1) == 0 && me < n / 2 ? 1 : 0);
 #pragma unroll 2
-    for (int e = me; e < npairs; e += G) {
-        const uint32_t rc = ptab[e];
-        const int r = rc & 0xffff, c = rc >> 16;
-        const cfloat u = fphasor(Cf[r * ld + c]);
-        const cfloat t = cconj(cmulc(cmul(u, wb[c]), wb[r]));
-        if (!cisnan(t)) {
-            sre += t.re;
-            sim += t.im;
-            cnt += 1.f;
+        for (int d = 1; d <= half; ++d) {
+            int j = me + d;
+            const bool wrap = j >= n;
+            j = wrap ? j - n : j;
+            const float xr = cr[j], xi = ci[j], wr = U[j], wi = U[KB + j];
+            const float s = rsqrtf(xr * xr + xi * xi);
+            const float ur = xr * wr - xi * wi, ui = xr * wi + xi * wr;
+            const float t = wrap ? -s : s;
+            pr = fmaf(s, ur, pr);
+            pi = fmaf(s, ui, pi);
+            qr = fmaf(t, ur, qr);
+            qi = fmaf(t, ui, qi);
         }
+        sre = w.re * pr + w.im * pi;
+        sim = w.re * qi - w.im * qr;
     }
     sre = gr.sum(sre);
     sim = gr.sum(sim);
-    cnt = gr.sum(cnt);  // exact: at most 2016 pairs
+    if (a.baseline_lag > 0 || isnan(sre + sim)) {
+        sre = sim = cnt = 0.f;
+#pragma unroll 1
+        for (int e = me; e < npairs; e += G) {
+            const uint32_t rc = ptab[e];
+            const int r = rc & 0xff, c = rc >> 8;
+            const cfloat u = fphasor(cmake(Cr[r * LD + c], Ci[r * LD + c]));
+            const cfloat t = cconj(cmulc(cmul(u, cmake(U[c], U[KB + c])), cmake(U[r], U[KB + r])));
+            if (!cisnan(t)) {
+                sre += t.re;
+                sim += t.im;
+                cnt += 1.f;
+            }
+        }
+        sre = gr.sum(sre);
+        sim = gr.sum(sim);
+        cnt = gr.sum(cnt);  // exact: at most 2016 pairs
+    }
     if (me == 0) {
         const float tc = hypotf(sre / cnt, sim / cnt);
         a.tcoh[p] = isfinite(tc) ? tc : 0.f;
     }
-    gr.sync();
 }
 
 // Solve-only pass over all pixels with the register solver (n <= K), one pixel per
-// group of G warps.  The coherence comes planar (diagonal, then (Re, Im) of the
+// group of G threads.  The coherence comes planar (diagonal, then (Re, Im) of the
 // lower pair (i, j), i > j, at o = i(i-1)/2 + j) or as full (npix, n, n) matrices
 // of which the lower triangle is read.
 // Two CTAs per SM (128 registers) wherever two CTAs' shared memory fits, K <= 46: the
-// two-warp instances would take 150-250 registers and one CTA; bounded, K <= 46 compiles
-// without spills and runs 14-16 % faster at N = 36-45.
+// two-warp instances would take more registers and one CTA.
 template <int K, int G>
-__global__ void __launch_bounds__(256, (G == 64 && K > 46) ? 1 : 2) k_solve_reg(PixArgs a, RegLayout L) {
-    extern __shared__ __align__(16) unsigned char reg_smem[];
+__global__ void __launch_bounds__(256, (G == 64 && K > 46) ? 1 : 2) k_solve_reg(PixArgs a) {
+    using S = RegShape<K, G>;
+    constexpr int LD = S::LD;
+    extern __shared__ __align__(16) float reg_smem[];
     const int warp = threadIdx.x >> 5;
     Grp<G> gr;
     gr.lane = threadIdx.x & 31;
@@ -483,77 +668,89 @@ __global__ void __launch_bounds__(256, (G == 64 && K > 46) ? 1 : 2) k_solve_reg(
         gr.gl = gr.wig * 32 + gr.lane;
         gr.bar = 1 + group;
     }
-    unsigned char* base = reg_smem + group * L.bytes;
-    gr.x = reinterpret_cast<float*>(base + L.off_x);
-    cfloat* Cf = reinterpret_cast<cfloat*>(base + L.off_C);
-    float* Gs = reinterpret_cast<float*>(base + L.off_G);
-    cfloat* cb = reinterpret_cast<cfloat*>(base + L.off_b);
-    cfloat* wb = reinterpret_cast<cfloat*>(base + L.off_w);
-    uint32_t* ptab = reinterpret_cast<uint32_t*>(reg_smem + ngroups * L.bytes);  // shared by the CTA
-    const int n = a.n, ld = L.ld, lag = a.baseline_lag, me = gr.gl;
-    for (int o = threadIdx.x; o < n * (n - 1) / 2; o += blockDim.x) {
+    float* Cr = reg_smem + group * S::FLOATS;
+    float* Ci = Cr + S::PLANE;
+    float* Gs = Ci + S::PLANE;
+    float* U = Cr + S::OFF_U;
+    gr.x = Cr + S::OFF_X;
+    uint16_t* ptab = reinterpret_cast<uint16_t*>(reg_smem + ngroups * S::FLOATS);  // shared by the CTA: r | c << 8
+    const int n = a.n, lag = a.baseline_lag, me = gr.gl;
+    const int npairs = n * (n - 1) / 2;
+    for (int i = threadIdx.x; i < ngroups * S::FLOATS; i += blockDim.x) reg_smem[i] = 0.f;  // the padding stays 0
+    for (int o = threadIdx.x; o < npairs; o += blockDim.x) {
         int r = (int)((sqrtf(8.f * o + 1.f) + 1.f) * 0.5f);  // o = r(r-1)/2 + c, 0 <= c < r
         while (r * (r - 1) / 2 > o) --r;
         while ((r + 1) * r / 2 <= o) ++r;
-        ptab[o] = (uint32_t)r | ((uint32_t)(o - r * (r - 1) / 2) << 16);
+        ptab[o] = (uint16_t)(r | (o - r * (r - 1) / 2) << 8);
     }
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * ngroups;
-    bool staged = false;  // Gs holds this pixel's planar coherence (prefetched)
-    for (int64_t p = (int64_t)blockIdx.x * ngroups + group; p < a.npix; p += stride) {
+    RegFetch<K, G> in;
+    int64_t p = (int64_t)blockIdx.x * ngroups + group;
+    if (p < a.npix) in.load(a, p, ptab, me);
+    for (; p < a.npix; p += stride) {
         gr.sync();
+        // the planar sums are unnormalised: C_ij = numer_ij r_i r_j with r = 1 / sqrt(amp)
+        // (amp = the diagonal sum), 0 where r_i r_j >= 1e6 (covariance.py:131-142)
         if (a.Cplanar) {
-            if (staged) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            const float rme = me < n ? __frsqrt_rn(in.d.x) : 0.f;
+            if (me < n) U[me] = rme;
             gr.sync();
-            const float* src = staged ? Gs : a.Cplanar + p * n * n;
-            // the planar sums are unnormalised: C_ij = numer_ij r_i r_j with r = 1 / sqrt(amp)
-            // (amp = the diagonal sum), 0 where r_i r_j >= 1e6 (covariance.py:131-142)
-            float* rv = reinterpret_cast<float*>(wb);
-            const float rme = me < n ? __frsqrt_rn(src[me]) : 0.f;
-            if (me < n) rv[me] = rme;
-            gr.sync();
-            if (me < n) {
-                const float f = rme * rme;
-                Cf[me * ld + me] = cmake(f < 1e6f ? src[me] * f : 0.f, 0.f);
+            const float f = rme * rme;
+            in.d.x = f < 1e6f ? in.d.x * f : 0.f;
+        }
+        if (me < n) {
+            Cr[me * LD + me] = in.d.x;
+            Ci[me * LD + me] = in.d.y;
+        }
+#pragma unroll
+        for (int i = 0; i < S::NP; ++i) {
+            const int e = me + i * G;
+            if (e < npairs) {
+                const uint32_t rc = ptab[e];
+                const int r = rc & 0xff, c = rc >> 8;
+                cfloat v = cmake(in.v[i].x, in.v[i].y);
+                if (a.Cplanar) {
+                    const float f = U[r] * U[c];
+                    v = f < 1e6f ? cscale(v, f) : cmake(0.f, 0.f);
+                }
+                Cr[r * LD + c] = v.re;
+                Ci[r * LD + c] = v.im;
+                Cr[c * LD + r] = v.re;
+                Ci[c * LD + r] = -v.im;
+                const float gm = s_abs_approx(v);
+                Gs[r * LD + c] = gm;
+                Gs[c * LD + r] = gm;
             }
-            const int npairs = n * (n - 1) / 2;
-#pragma unroll 2
+        }
+        // options that few runs use, apart from the unrolled code: the baseline lag, and
+        // |Gamma| with a beta or a zero-correlation threshold
+        if (lag > 0 || a.beta_on || a.zct > 0.f) {
+#pragma unroll 1
             for (int e = me; e < npairs; e += G) {
                 const uint32_t rc = ptab[e];
-                const int r = rc & 0xffff, c = rc >> 16;
-                const float f = rv[r] * rv[c];
-                cfloat v = f < 1e6f ? cmake(src[n + 2 * e] * f, src[n + 2 * e + 1] * f) : cmake(0.f, 0.f);
-                if (lag > 0 && r - c >= lag) v = cmake(0.f, 0.f);
-                Cf[r * ld + c] = v;
-                Cf[c * ld + r] = cconj(v);
-            }
-        } else {
-            const cfloat* src = a.Cin + p * n * n;
-            for (int i = 0; i < n; ++i) {
-                if (me <= i) {
-                    cfloat c = src[i * n + me];
-                    if (lag > 0 && i - me >= lag) c = cmake(0.f, 0.f);
-                    Cf[i * ld + me] = c;
-                    if (me < i) Cf[me * ld + i] = cconj(c);
-                }
+                const int r = rc & 0xff, c = rc >> 8;
+                if (lag > 0 && r - c >= lag) Cr[r * LD + c] = Ci[r * LD + c] = Cr[c * LD + r] = Ci[c * LD + r] = 0.f;
+                const float gm = s_gamma(a, cmake(Cr[r * LD + c], Ci[r * LD + c]), false);
+                Gs[r * LD + c] = gm;
+                Gs[c * LD + r] = gm;
             }
         }
         gr.sync();
-        const float* next = a.Cplanar && p + stride < a.npix ? a.Cplanar + (p + stride) * n * n : nullptr;
-        solve_pixel_reg<K, G>(a, p, Cf, Gs, ld, cb, wb, ptab, next, gr);
-        staged = next != nullptr;
+        const int64_t next = p + stride;
+        solve_pixel_reg<K, G>(a, p, Cr, Ci, Gs, U, ptab, gr, [&]() {
+            in.load(a, next < a.npix ? next : p, ptab, me);  // unconditional: the old values die here
+        });
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // Host launch of the instance with K slots and G threads per pixel: 8 warps per CTA,
 // 256 / G pixel groups; a persistent grid of at most 8 waves.
 template <int K, int G>
 dpl_status launch_solve_reg_k(const PixArgs& a, cudaStream_t s) {
-    const RegLayout L = make_reg_layout(a.n);
     const int warps = 8;
     const int groups = warps * 32 / G;
-    const size_t smem = (size_t)groups * L.bytes + (size_t)a.n * (a.n - 1) / 2 * sizeof(uint32_t);
+    const size_t smem = (size_t)groups * RegShape<K, G>::FLOATS * sizeof(float) + (size_t)a.n * (a.n - 1) / 2 * sizeof(uint16_t);
     if (smem > 227 * 1024) return fail(DPL_ERR_UNSUPPORTED, "register solver: shared memory exceeds the SM limit");
     int dev = 0, sms = 0;
     DPL_CUDA_TRY(cudaGetDevice(&dev));
@@ -563,7 +760,7 @@ dpl_status launch_solve_reg_k(const PixArgs& a, cudaStream_t s) {
     DPL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve_reg<K, G>, warps * 32, smem));
     const int64_t resident = (int64_t)std::max(1, per_sm) * std::max(1, sms);
     const int64_t grid = std::min<int64_t>((a.npix + groups - 1) / groups, resident * 8);
-    k_solve_reg<K, G><<<(unsigned)std::max<int64_t>(grid, 1), warps * 32, smem, s>>>(a, L);
+    k_solve_reg<K, G><<<(unsigned)std::max<int64_t>(grid, 1), warps * 32, smem, s>>>(a);
     return check_launch("k_solve_reg");
 }
 
