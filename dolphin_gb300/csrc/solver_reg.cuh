@@ -48,6 +48,7 @@ __device__ __forceinline__ float f2_lo(f2 v) { return v.x; }
 __device__ __forceinline__ float f2_hi(f2 v) { return v.y; }
 __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ f2 f2_neg(f2 v) { return make_float2(-v.x, -v.y); }  // an operand modifier
 __device__ __forceinline__ f2 f2_ld(const float* p, int q) { return reinterpret_cast<const float2*>(p)[q]; }
 __device__ __forceinline__ void f2_ld2(const float* p, int q, f2& a, f2& b) {  // pairs 2q, 2q + 1
     const float4 t = reinterpret_cast<const float4*>(p)[q];
@@ -161,7 +162,7 @@ __device__ __forceinline__ bool r_sweep(f2 (&g)[K / 2], float* buf, const Grp<G>
             // a_kj - (1 - 1/p) a_kj so that every thread runs the same FMA
             const float t = me ? 1.f - ip : g0 * ip;
             const float last = me ? -ip : g0 * ip;
-            const f2 nt = f2_pack(-t, -t);
+            const f2 nt = f2_neg(f2_pack(t, t));
 #pragma unroll
             for (int q = 0; q < K / 4; ++q) {
                 f2 x, y;
@@ -183,7 +184,7 @@ __device__ __forceinline__ bool r_sweep(f2 (&g)[K / 2], float* buf, const Grp<G>
             const bool me = gr.gl == k + 1;
             const float t = me ? 1.f - ip : g1 * ip;
             const float last = me ? -ip : g1 * ip;
-            const f2 nt = f2_pack(-t, -t);
+            const f2 nt = f2_neg(f2_pack(t, t));
             f2 first = f2_pack(0.f, 0.f);
 #pragma unroll
             for (int q = 0; q < K / 4; ++q) {
@@ -226,11 +227,11 @@ __device__ __forceinline__ bool r_sweep_c(f2 (&re)[K / 2], f2 (&im)[K / 2], floa
             const bool me = gr.gl == k;
             const float sr = a0 * ip, si = c0 * ip;
             const float tr = me ? 1.f - ip : sr, ti = me ? 0.f : si;
-            const f2 ntr = f2_pack(-tr, -tr), nti = f2_pack(-ti, -ti), ptr = f2_pack(tr, tr);
+            const f2 ptr = f2_pack(tr, tr), pti = f2_pack(ti, ti);
             // slot s: a_ij - t a_kj, a_kj = conj(buffer entry s)
             auto update = [&](int q, f2 br, f2 bi) {
-                re[q] = f2_fma(ntr, br, f2_fma(nti, bi, re[q]));
-                im[q] = f2_fma(nti, br, f2_fma(ptr, bi, im[q]));
+                re[q] = f2_fma(f2_neg(ptr), br, f2_fma(f2_neg(pti), bi, re[q]));
+                im[q] = f2_fma(f2_neg(pti), br, f2_fma(ptr, bi, im[q]));
             };
 #pragma unroll
             for (int q = 0; q < K / 4; ++q) {
@@ -258,11 +259,11 @@ __device__ __forceinline__ bool r_sweep_c(f2 (&re)[K / 2], f2 (&im)[K / 2], floa
             const bool me = gr.gl == k + 1;
             const float sr = a1 * ip, si = c1 * ip;
             const float tr = me ? 1.f - ip : sr, ti = me ? 0.f : si;
-            const f2 ntr = f2_pack(-tr, -tr), nti = f2_pack(-ti, -ti), ptr = f2_pack(tr, tr);
+            const f2 ptr = f2_pack(tr, tr), pti = f2_pack(ti, ti);
             f2 fr = f2_pack(0.f, 0.f), fi = f2_pack(0.f, 0.f);
             auto update = [&](int q, f2 br, f2 bi) {  // pair q into pair q - 1
-                const f2 x = f2_fma(ntr, br, f2_fma(nti, bi, re[q]));
-                const f2 y = f2_fma(nti, br, f2_fma(ptr, bi, im[q]));
+                const f2 x = f2_fma(f2_neg(ptr), br, f2_fma(f2_neg(pti), bi, re[q]));
+                const f2 y = f2_fma(f2_neg(pti), br, f2_fma(ptr, bi, im[q]));
                 if (q == 0) {
                     fr = x;
                     fi = y;
@@ -290,7 +291,7 @@ __device__ __forceinline__ bool r_sweep_c(f2 (&re)[K / 2], f2 (&im)[K / 2], floa
     return !bad;
 }
 
-// Publishes a vector as three planes (Re, Im, -Im) of KB floats.
+// Publishes a vector as two planes (Re, Im) of KB floats.
 template <int K, int G>
 __device__ __forceinline__ void r_publish(float* vb, cfloat x, const Grp<G>& gr) {
     constexpr int KB = RegShape<K, G>::KB;
@@ -298,7 +299,6 @@ __device__ __forceinline__ void r_publish(float* vb, cfloat x, const Grp<G>& gr)
     if (gr.gl < K) {
         vb[gr.gl] = x.re;
         vb[KB + gr.gl] = x.im;
-        vb[2 * KB + gr.gl] = -x.im;
     }
     gr.sync();
 }
@@ -311,20 +311,19 @@ __device__ __forceinline__ cfloat r_matvec(const f2 (&hr)[K / 2], const f2 (&hi)
     constexpr int KB = RegShape<K, G>::KB;
     r_publish<K, G>(vb, x, gr);
     f2 ar = f2_pack(0.f, 0.f), ai = f2_pack(0.f, 0.f);
-    auto step = [&](int q, f2 r, f2 i, f2 n) {
-        ar = f2_fma(hr[q], r, f2_fma(hi[q], n, ar));
+    auto step = [&](int q, f2 r, f2 i) {
+        ar = f2_fma(hr[q], r, f2_fma(hi[q], f2_neg(i), ar));
         ai = f2_fma(hr[q], i, f2_fma(hi[q], r, ai));
     };
 #pragma unroll
     for (int q = 0; q < K / 4; ++q) {
-        f2 r0, r1, i0, i1, n0, n1;
+        f2 r0, r1, i0, i1;
         f2_ld2(vb, q, r0, r1);
         f2_ld2(vb + KB, q, i0, i1);
-        f2_ld2(vb + 2 * KB, q, n0, n1);
-        step(2 * q, r0, i0, n0);
-        step(2 * q + 1, r1, i1, n1);
+        step(2 * q, r0, i0);
+        step(2 * q + 1, r1, i1);
     }
-    if (K % 4) step(K / 2 - 1, f2_ld(vb, K / 2 - 1), f2_ld(vb + KB, K / 2 - 1), f2_ld(vb + 2 * KB, K / 2 - 1));
+    if (K % 4) step(K / 2 - 1, f2_ld(vb, K / 2 - 1), f2_ld(vb + KB, K / 2 - 1));
     if (gr.gl >= K) return cmake(0.f, 0.f);  // lanes beyond the matrix
     return cmake(f2_lo(ar) + f2_hi(ar), f2_lo(ai) + f2_hi(ai));
 }
@@ -558,7 +557,7 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
             const f2 gq = f2_ld(Gi, q);
             const f2 hr = f2_mul(f2_ld(cr, q), gq), hi = f2_mul(f2_ld(ci, q), gq);
             const f2 xr = f2_ld(U, q), xi = f2_ld(U + KB, q);
-            ar = f2_fma(hr, xr, f2_fma(hi, f2_ld(U + 2 * KB, q), ar));
+            ar = f2_fma(hr, xr, f2_fma(hi, f2_neg(xi), ar));
             ai = f2_fma(hr, xi, f2_fma(hi, xr, ai));
         }
         const cfloat acc = row ? cmake(f2_lo(ar) + f2_hi(ar), f2_lo(ai) + f2_hi(ai)) : cmake(0.f, 0.f);
