@@ -201,6 +201,12 @@ __device__ void warp_covariance(const PixArgs& a, int64_t p, cfloat* C, cfloat* 
     if (count_out) *count_out = count;
 }
 
+}  // namespace dpl
+
+#include "cov_simt.cuh"
+
+namespace dpl {
+
 template <int NB, int MODE, bool kLU>
 __global__ void __launch_bounds__(256) k_pixel(PixArgs a) {
     extern __shared__ __align__(16) unsigned char pix_smem[];
@@ -215,9 +221,9 @@ __global__ void __launch_bounds__(256) k_pixel(PixArgs a) {
     m.d = reinterpret_cast<float*>(base + a.off_d);
     m.piv = reinterpret_cast<int*>(base + a.off_piv);
     const int n = a.n;
-    const int64_t total = kLU ? (int64_t)*a.list_count : a.npix;
+    const int64_t total = a.list ? (int64_t)*a.list_count : a.npix;
     for (int64_t idx = (int64_t)blockIdx.x * nwarps + warp; idx < total; idx += (int64_t)gridDim.x * nwarps) {
-        const int64_t p = kLU ? (int64_t)a.list[idx] : idx;
+        const int64_t p = a.list ? (int64_t)a.list[idx] : idx;
         if (MODE == kSolveOnly) {
             __syncwarp();
             if (a.Cplanar) {
@@ -554,7 +560,7 @@ static dpl_status launch_pixel_pass(const PixArgs& a, cudaStream_t s) {
         int per_sm = 0;
         DPL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem));
         const int64_t resident = (int64_t)std::max(1, per_sm) * std::max(1, sms);
-        int64_t grid = kLU ? resident : std::min<int64_t>((a.npix + warps - 1) / warps, resident * 8);
+        int64_t grid = a.list ? resident : std::min<int64_t>((a.npix + warps - 1) / warps, resident * 8);
         kernel<<<(unsigned)std::max<int64_t>(grid, 1), warps * 32, smem, s>>>(a);
         return check_launch(kLU ? "k_pixel (LU pass)" : "k_pixel");
     };
@@ -995,9 +1001,41 @@ static dpl_status pl_finish(PlState& S, cudaStream_t s, bool cov_done) {
         st = timed(s, 1, [&] {
             return launch_pixel<kSolveOnly>(a, s, w.fb, P.nonconverged_mode == 0 ? w.nc : nullptr);
         });
+    } else if (w.Cg) {
+        // window or strides too large for the tensor-core tiles: float32 covariance on the
+        // CUDA cores and the register solver on it, its last iterate kept as in the plain
+        // form.  Its explicit inverses cost accuracy where a pixel is ill-conditioned: those
+        // few pixels, and the undecided ones (|Gamma| not positive definite), are listed and
+        // solved by the plain form, then the LU pass takes what both listed.
+        // 512 x 384 outputs, strides 3 x 6, 11 x 23 window, N = 21: 21.1 -> 6.4 ms on the device
+        // (the fused k_pixel took 20.6 ms; k_cov_simt 4.0, k_solve_reg 1.5, the list 0.3).
+        st = timed(s, 0, [&] { return launch_cov_simt<1>(cov_simt_block(n), a, w.Cg, s); });
+        if (st != DPL_OK) return st;
+        st = timed(s, 1, [&]() -> dpl_status {
+            DPL_CUDA_TRY(cudaMemsetAsync(w.fb, 0, sizeof(int), s));
+            DPL_CUDA_TRY(cudaMemsetAsync(w.nc, 0, sizeof(int), s));
+            a.fb_count = w.fb;
+            a.fb_list = w.fb + 64;
+            a.nc_flag = nullptr;
+            PixArgs b = a;
+            b.Cplanar = w.Cg;
+            b.planar_norm = 1;
+            b.ill_count = w.nc;
+            b.ill_list = w.nc + 64;
+            dpl_status e = launch_solve_reg(b, s);
+            if (e != DPL_OK) return e;
+            PixArgs c = a;
+            c.list = b.ill_list;
+            c.list_count = b.ill_count;
+            e = launch_pixel_pass<kFused, false>(c, s);
+            if (e != DPL_OK) return e;
+            fill_pix_layout(c, n, 2 * P.hx + 1, true);
+            c.list = a.fb_list;
+            c.list_count = a.fb_count;
+            return launch_pixel_pass<kFused, true>(c, s);
+        });
     } else {
-        // plain form (or a window too large for the tensor-core tiles): SIMT covariance
-        // fused with the solver
+        // plain form: SIMT covariance fused with the solver
         st = timed(s, 0, [&] { return launch_pixel<kFused>(a, s, w.fb); });
     }
     if (st != DPL_OK) return st;

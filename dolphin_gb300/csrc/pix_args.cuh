@@ -61,6 +61,7 @@ struct PixArgs {
     const cfloat* vstart;    // optional EMI starting vectors (npix, n); plain start when null
     int16_t* iters;          // optional: eigen-iterations used per pixel (npix)
     const float* Cplanar;    // solve-only input, planar per pixel: diagonal | (Re, Im) per lower pair
+    int planar_norm;         // Cplanar is normalised already (else raw sums)
     int use_evd, beta_on;
     float one_minus_beta, beta, zct;
     int ref_idx, compute_crlb, crlb_ref, baseline_lag;
@@ -76,8 +77,10 @@ struct PixArgs {
     int32_t* counts;         // (npix) or null
     int* fb_list;            // pixels whose EMI shifted matrix is indefinite (for the LU pass)
     int* fb_count;
-    const int* list;         // LU pass: pixels list[0 .. *list_count)
+    const int* list;         // k_pixel: pixels list[0 .. *list_count) instead of all (always so in the LU pass)
     const int* list_count;
+    int* ill_list;           // register solver: ill-conditioned pixels for the plain form (null: not listed)
+    int* ill_count;
     int lanes;               // register solver: threads per pixel (8, 16, 32; 0 = the smallest that fits)
     int* nc_list;            // pixels whose eigen-iteration missed its stopping rule (null: not listed)
     int* nc_count;

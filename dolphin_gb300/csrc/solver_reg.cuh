@@ -387,7 +387,7 @@ __device__ __forceinline__ float r_iterate(cfloat& v, const Grp<G>& gr, int& ste
 
 // Full solve for one pixel whose Hermitian coherence matrix is in the planes Cr, Ci (both
 // triangles) and whose |Gamma| is in Gs off the diagonal.  A pixel whose shifted EMI
-// matrix is not positive definite is appended to a.fb_list and left for the LU pass.
+// matrix is not positive definite is listed and left for the LU pass (or the plain form).
 // `fetch` loads the group's next pixel.
 template <int K, int G, class Fetch>
 __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, float* Cr, float* Ci, float* Gs, float* U,
@@ -519,7 +519,11 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
             cr[me] = cd;
         }
         if (!r_sweep_c<K, G>(re, im, U, gr)) {
-            if (me == 0) a.fb_list[atomicAdd(a.fb_count, 1)] = (int)p;
+            // not positive definite: the LU pass, or the plain form's own decision
+            if (me == 0) {
+                if (a.ill_list) a.ill_list[atomicAdd(a.ill_count, 1)] = (int)p;
+                else a.fb_list[atomicAdd(a.fb_count, 1)] = (int)p;
+            }
             fetch();
             return;
         }
@@ -544,6 +548,14 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
     if (!(diff <= 1e-5f) && warm) {  // a warm start that misses the rule (or goes NaN): plain EMI
         v = row ? cmake(1.f / sqrtf((float)n), 0.f) : cmake(0.f, 0.f);
         diff = r_iterate<G>(v, gr, steps, op);
+    }
+    // ill-conditioned for the explicit inverses, or not decided by them: listed for the
+    // plain form.  Of 160 k pixels at N = 45 (11 x 23 windows over parcels of different
+    // coherence) every phase that came out more than 1e-4 rad from the plain form's had a
+    // diagonal entry of |Gamma|^{-1} above 50 or more than 45 steps; 0.1 % are listed.
+    if (a.ill_list && !a.use_evd) {
+        const bool ill = gr.any(row && gd > 32.f);
+        if ((evd || ill || steps > 24) && me == 0) a.ill_list[atomicAdd(a.ill_count, 1)] = (int)p;
     }
     // 49 steps without meeting the stopping rule (a NaN difference stops the loop, as in
     // the reference): listed for the dense eigensolver
@@ -691,7 +703,8 @@ __global__ void __launch_bounds__(256, (G == 64 && K > 46) ? 1 : 2) k_solve_reg(
         gr.sync();
         // the planar sums are unnormalised: C_ij = numer_ij r_i r_j with r = 1 / sqrt(amp)
         // (amp = the diagonal sum), 0 where r_i r_j >= 1e6 (covariance.py:131-142)
-        if (a.Cplanar) {
+        const bool raw = a.Cplanar && !a.planar_norm;
+        if (raw) {
             const float rme = me < n ? __frsqrt_rn(in.d.x) : 0.f;
             if (me < n) U[me] = rme;
             gr.sync();
@@ -709,7 +722,7 @@ __global__ void __launch_bounds__(256, (G == 64 && K > 46) ? 1 : 2) k_solve_reg(
                 const uint32_t rc = ptab[e];
                 const int r = rc & 0xff, c = rc >> 8;
                 cfloat v = cmake(in.v[i].x, in.v[i].y);
-                if (a.Cplanar) {
+                if (raw) {
                     const float f = U[r] * U[c];
                     v = f < 1e6f ? cscale(v, f) : cmake(0.f, 0.f);
                 }
