@@ -14,11 +14,17 @@ def torch():
     return _t
 
 
+_cuda = None  # torch, once a CUDA device was found (asking again costs 3 us, 26 times per block)
+
+
 def require_cuda():
-    t = torch()
-    if not t.cuda.is_available():
-        raise RuntimeError("dolphin_gb300 needs a CUDA GPU (there is no CPU fallback)")
-    return t
+    global _cuda
+    if _cuda is None:
+        t = torch()
+        if not t.cuda.is_available():
+            raise RuntimeError("dolphin_gb300 needs a CUDA GPU (there is no CPU fallback)")
+        _cuda = t
+    return _cuda
 
 
 def is_device_tensor(x) -> bool:

@@ -820,6 +820,8 @@ static void set_solver_params(PixArgs& a, int use_evd, double beta, double zct, 
     a.crlb_factor_d = 2.0 * num_looks;
 }
 
+constexpr size_t kPlStatusBytes = 256 + 64;
+
 struct PlWorkspace {
     int* status;
     unsigned int* valid_bits;
@@ -838,7 +840,7 @@ static size_t pl_workspace_layout(int64_t n, int64_t rows, int64_t cols, int sy,
     Workspace ws{base, ~size_t(0)};
     const int64_t npix = rows * cols, P = (rows / sy) * (cols / sx);
     PlWorkspace t{};
-    t.status = ws.take<int>(16);
+    t.status = ws.take<int>(16);  // the first kPlStatusBytes hold the status and the valid bits
     t.valid_bits = ws.take<unsigned int>(16);
     t.Cg = cov_form == 0 || cov_form == 3 ? ws.take<float>(P * n * n) : nullptr;
     t.fb = ws.take<int>(P + 64);
@@ -918,8 +920,7 @@ static dpl_status pl_begin(const dpl_pl_params* prm, const dpl_pl_inputs* in, co
     S.out_rows = (int)(P.rows / P.sy);
     S.out_cols = (int)(P.cols / P.sx);
     S.Pout = (int64_t)S.out_rows * S.out_cols;
-    DPL_CUDA_TRY(cudaMemsetAsync(w.status, 0, 64, s));
-    DPL_CUDA_TRY(cudaMemsetAsync(w.valid_bits, 0, 64, s));
+    DPL_CUDA_TRY(cudaMemsetAsync(w.status, 0, kPlStatusBytes, s));
     {
         size_t smem = (size_t)kPrepPix * (n + 1) * sizeof(cfloat);
         DPL_CUDA_TRY(cudaFuncSetAttribute(k_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1097,11 +1098,15 @@ static dpl_status pl_decode(int n, const int* status, const unsigned int* valid)
 
 // Waits for `stream`, then reports what the enqueued pipeline left in the workspace.
 static dpl_status pl_check(int n, const PlWorkspace& w, cudaStream_t s) {
-    int host_status[2] = {0, 0};
-    unsigned int host_valid[2] = {0, 0};
-    DPL_CUDA_TRY(cudaMemcpyAsync(host_status, w.status, sizeof(int), cudaMemcpyDeviceToHost, s));
-    DPL_CUDA_TRY(cudaMemcpyAsync(host_valid, w.valid_bits, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+    // the two words lie one behind the other at the head of the workspace: one copy
+    char host[kPlStatusBytes];
+    DPL_CUDA_TRY(cudaMemcpyAsync(host, w.status, kPlStatusBytes, cudaMemcpyDeviceToHost, s));
     DPL_CUDA_TRY(cudaStreamSynchronize(s));
+    int host_status[1];
+    unsigned int host_valid[2];
+    std::memcpy(host_status, host, sizeof host_status);
+    std::memcpy(host_valid, host + (reinterpret_cast<char*>(w.valid_bits) - reinterpret_cast<char*>(w.status)),
+                sizeof host_valid);
     return pl_decode(n, host_status, host_valid);
 }
 

@@ -552,6 +552,31 @@ size_t dpl::ks_workspace_size(int64_t nslc, int64_t rows, int64_t cols) {
            align_up((size_t)nslc * rows * cols * sizeof(float), 256);
 }
 
+// shp/_ks.py:221-239: distances from 0.01 in steps of 0.001, the first whose Kolmogorov
+// series (100 terms, n / 2 effective samples) is <= alpha.  The reference's operations in
+// its order, so the distance is the same double: the power of two of `value` through pow()
+// and the terms through exp(), as its interpreter evaluates them.  Host code: as a Python
+// loop the scan took 4-7 ms a call, longer than the kernels.
+extern "C" double dpl_ks_critical_distance(int64_t nslc, double alpha) {
+    const double n_eff = (double)nslc / 2.0, sq = std::sqrt(n_eff);
+    double cur = 0.01;
+    while (cur <= 1.0) {
+        const double value = cur * (sq + 0.12 + 0.11 / sq);
+        const double scale = -2 * std::pow(value, 2.0);
+        double pvalue = 0.0;
+        for (int t = 1; t <= 100; ++t) {
+            const double term = std::exp(scale * (double)(t * t));
+            // the terms fall: below a quarter of the last place none changes the sum
+            if (term <= pvalue * 0x1p-55) break;
+            pvalue = t & 1 ? pvalue + term : pvalue - term;
+        }
+        pvalue = std::max(0.0, std::min(1.0, 2 * pvalue));
+        if (pvalue <= alpha) return cur;
+        cur += 0.001;
+    }
+    return 0.1;
+}
+
 extern "C" size_t dpl_shp_ks_workspace_size(int64_t nslc, int64_t rows, int64_t cols) {
     return ks_workspace_size(nslc, rows, cols);
 }

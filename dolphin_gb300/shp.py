@@ -18,10 +18,11 @@ __all__ = ["estimate_neighbors", "glrt_threshold", "ks_critical_distance"]
 
 
 def glrt_threshold(alpha: float) -> float:
-    """chi-square(1) quantile at 1 - alpha (shp/_glrt.py:78)."""
-    from scipy import stats
+    """chi-square(1) quantile at 1 - alpha (shp/_glrt.py:78): what ``chi2.ppf`` evaluates,
+    without its argument checks (48 us a call)."""
+    from scipy.special import gammaincinv
 
-    return float(stats.chi2.ppf(1 - alpha, df=1))
+    return float(2 * gammaincinv(0.5, 1 - alpha))
 
 
 def ks_critical_distance(nslc: int, alpha: float) -> float:
@@ -30,21 +31,8 @@ def ks_critical_distance(nslc: int, alpha: float) -> float:
     Scans distances from 0.01 in steps of 0.001 and returns the first whose
     Kolmogorov-series p-value (100 terms, N/2 effective samples) is <= alpha.
     """
-    n_eff = nslc / 2.0
-    cur = 0.01
-    crit = 0.1
-    sq = math.sqrt(n_eff)
-    while cur <= 1.0:
-        value = cur * (sq + 0.12 + 0.11 / sq)
-        pvalue = 0
-        for t in range(1, 101):
-            pvalue += ((-1) ** (t - 1)) * math.exp(-2 * (value**2) * (t**2))
-        pvalue = max(0.0, min(1.0, 2 * pvalue))
-        if pvalue <= alpha:
-            crit = cur
-            break
-        cur += 0.001
-    return crit
+    0.11 / math.sqrt(nslc / 2.0)  # raises for nslc <= 0, as the reference does
+    return float(_lib.load().dpl_ks_critical_distance(int(nslc), float(alpha)))
 
 
 def _method_name(method) -> str:

@@ -101,3 +101,21 @@ def test_glrt_masks(nslc, alpha, hw, strides):
         bad = O.estimate_neighbors_glrt(mean, np.where(neg > 0, np.nan, var), hw, strides, nslc, alpha, exact=True)
         want = want & bad
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("alpha", [0.5, 0.05, 0.01, 0.001, 1e-9])
+def test_ks_critical_distance_is_the_scan(alpha):
+    from dolphin_gb300 import _build
+    from dolphin_gb300.shp import ks_critical_distance
+
+    _build.build_library()
+    for n in [1, 2, 3, 5, 10, 17, 30, 45, 64, 300]:
+        assert ks_critical_distance(n, alpha) == O.ks_critical_distance(n, alpha)
+
+
+def test_glrt_threshold_is_the_quantile():
+    stats = pytest.importorskip("scipy.stats")
+    from dolphin_gb300.shp import glrt_threshold
+
+    for alpha in [0.0, 1e-12, 1e-5, 0.001, 0.01, 0.05, 0.3, 0.9, 1.0]:
+        assert glrt_threshold(alpha) == float(stats.chi2.ppf(1 - alpha, df=1))
