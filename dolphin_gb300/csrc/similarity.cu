@@ -9,22 +9,31 @@
 //                invalid or masked gets NaN phasors: every similarity it takes part in is
 //                then NaN, which the summaries skip, exactly as the reference skips masked
 //                pixels (the count of usable neighbours only matters through "none").
-// k_similarity<H> -- persistent; a CTA of 512 threads owns a tile of pixels.  Eight
+// k_similarity<H> -- persistent; a CTA owns a tile of pixels.  Eight
 //                layers at a time of the tile's neighbourhood (tile + H on every side,
 //                edge pixels replicated: the reference clips each neighbour coordinate
 //                to the image) are staged in shared memory with cp.async, double-
-//                buffered across chunks and tiles.  A group of G >= 2H + 1 lanes owns P
-//                vertically adjacent pixels of one column; lane dc + H loads the
-//                2H + P staged values of column c + dc and accumulates, in registers and
-//                over all layers, the similarities of its P pixels with their 2H + 1
-//                neighbours in that column (each load serves P pixels).  The circle's
-//                K similarities of a pixel thus sit in the registers of its group, and
-//                the summary is taken there: the maximum by a group reduction, the
-//                median by a selection on order-preserving keys, each step one
-//                group-wide count (redux.sync) around an interpolated pivot.  The
-//                pixel itself (which
+//                buffered across chunks and tiles.  A group of G >= 2H + J lanes owns P
+//                vertically adjacent pixels of each of J adjacent columns c ..; lane l
+//                loads the 2H + P staged values of column c + l - H and accumulates, in
+//                registers and over all layers, the similarities of its J P pixels with
+//                their 2H + 1 neighbours in that column (each load serves J P pixels).
+//                The circle's K similarities of a pixel thus sit in the registers of its
+//                group.  The maximum is a group reduction.  For the median the K keys
+//                (order-preserving integers) go through the stage buffer just consumed to
+//                LP = 4 .. 16 lanes per pixel, without the square's corners and the idle
+//                lanes, so that a warp selects for as many pixels at once as fit; each
+//                step of the selection is one group-wide count (redux.sync) around an
+//                interpolated pivot.  The pixel itself (which
 //                a clipped offset reaches at the image edge) and NaN similarities are
 //                left out.
+//
+//                Bound by issue slots (64 % used at 12 warps per SM).  1400 x 1500 pixels,
+//                30 layers, with the prep: radius 7 median 3.98 -> 3.22 ms and maximum
+//                2.34 -> 1.90 ms, radius 11 median 9.59 -> 8.07 ms, against one column per
+//                group (five reads of the stage per pixel and layer instead of three, tiles
+//                of 16 x 4 instead of 16 x 12 pixels: 7 instead of 3.5 staged values per
+//                pixel) and a selection in the sums' registers for two pixels per warp.
 #include <algorithm>
 #include <cstdio>
 #include <utility>
@@ -224,29 +233,45 @@ struct SimArgs {
     int kind;            // 0 median, 1 max
     const float2* unit;  // (m, rows, cols)
     float* out;          // (rows, cols)
-    int hc[2 * kSimHMax + 1];  // half-height of column dc (at index dc + H)
+    int hc[2 * kSimHMax + 1];    // half-height of column dc (at index dc + H)
+    int base[2 * kSimHMax + 1];  // its first slot among the circle's K
+    int K;
 };
 
-// Work layout for largest offset H.  A group of G lanes (G >= 2H + 1) owns P vertically
-// adjacent pixels of one column; its lane dc + H accumulates their similarities with
-// the 2H + 1 neighbours in column c + dc.  A CTA owns TC x TR pixels.
+// neighbours of the circles of largest offset 1 .. 15
+constexpr int kSimCircle[kSimHMax + 1] = {0, 8, 20, 36, 68, 96, 136, 176, 220, 292, 348, 420, 488, 568, 664, 748};
+
+// Work layout for largest offset H.  A group of G lanes (G >= 2H + J) owns P vertically
+// adjacent pixels of J adjacent columns; its lane l accumulates their similarities with
+// the 2H + 1 neighbours of each in column c + l - H.  A CTA owns TC x TR pixels.
 template <int H>
 struct SimShape {
     static constexpr int D = 2 * H + 1;
     static constexpr int G = D <= 4 ? 4 : D <= 8 ? 8 : D <= 16 ? 16 : 32;
+    // two columns where a lane's 2 P D sums fit the registers; the widest circles keep one
+    static constexpr int J = G == 32 ? 1 : 2;
     static constexpr int P = H <= 10 ? 4 : 2;
     static constexpr int GPW = 32 / G;
-    // 256 threads (two CTAs per SM, which drift apart so that one accumulates while the
-    // other takes its summaries) except for the widest groups, whose tiles would be thin
-    static constexpr int THREADS = G == 32 ? 512 : 256;
+    static constexpr int THREADS = G == 32 ? 512 : 384;
     static constexpr int UNITS = THREADS / 32 * GPW;
     static constexpr int TC = G == 4 ? 32 : 16;
-    static constexpr int TR = UNITS / TC * P;
+    static constexpr int UC = TC / J;  // units across a tile
+    static constexpr int TR = UNITS / UC * P;
     static constexpr int TRH = TR + 2 * H, SW = TC + 2 * H;  // staged rows and columns
     static constexpr int LAYER = TRH * SW;                   // float2 per staged layer
     static constexpr int STAGE = kSimChunk * LAYER;
     static constexpr size_t SMEM = 2 * (size_t)STAGE * sizeof(float2);
-    static_assert(UNITS % TC == 0, "tile rows");
+    static_assert(UNITS % UC == 0, "tile rows");
+    static_assert(D + J - 1 <= G, "lanes");
+    // selection: PB pixel rows at a time, so NPX pixels per warp, LP lanes and KL keys per
+    // lane each; a pixel's keys are KP words apart (KP = LP mod 32: conflict-free loads)
+    static constexpr int PB = G == 32 && H <= 12 ? 2 : 1;
+    static constexpr int NPX = GPW * J * PB;
+    static constexpr int LP = 32 / NPX;
+    static constexpr int K = kSimCircle[H];
+    static constexpr int KL = (K + LP - 1) / LP;
+    static constexpr int KP = (KL * LP - LP + 31) / 32 * 32 + LP;
+    static_assert(P % PB == 0 && THREADS / 32 * NPX * KP * 4 <= STAGE * 8, "selection scratch");
 };
 
 __device__ __forceinline__ void sim_cp8(float2* dst, const float2* src, bool fill) {
@@ -265,8 +290,8 @@ __device__ __forceinline__ float sim_unkey(uint32_t k) {
 }
 
 // Reductions over the G-lane groups of a warp, executed by all 32 lanes together so
-// that no collective runs under divergence: sums through one warp-wide redux of
-// per-group bit fields (a group's sum never exceeds its field), minima and maxima
+// that no collective runs under divergence: sums (below 256 with G = 8) through one
+// warp-wide redux of per-group bit fields where these hold them, minima and maxima
 // through xor butterflies that stay inside each group.
 template <int G>
 struct SimGroup {
@@ -274,6 +299,11 @@ struct SimGroup {
     int shift;
     __device__ __forceinline__ explicit SimGroup(int lane) : shift((lane / G) * G) {}
     __device__ __forceinline__ int sum(int v) const {
+        if (G < 8) {
+#pragma unroll
+            for (int o = G / 2; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            return v;
+        }
         const unsigned t = __reduce_add_sync(0xffffffffu, (unsigned)v << shift);
         if (FW == 32) return (int)t;
         return (int)((t >> shift) & ((1u << (FW & 31)) - 1u));
@@ -301,7 +331,7 @@ __device__ __forceinline__ int sim_count_below(const uint32_t (&key)[D], uint32_
 
 // Key of rank k (0-based, among the group's n valid keys; a left-out entry has key 0,
 // below every key of a number, and a lane holds `zeros` of them) given that it lies in
-// [L, U], `below` valid keys are < L and `upto` are <= U.  Each step counts the valid
+// [L, U].  Each step counts the valid
 // keys below a pivot t with one group-wide reduction and keeps the side that holds rank
 // k.  The pivot interpolates the rank linearly in value between L and U (a pixel's
 // similarities are spread fairly evenly; about 7 steps for a median of 20 to 140), or
@@ -310,8 +340,9 @@ __device__ __forceinline__ int sim_count_below(const uint32_t (&key)[D], uint32_
 // are done.
 template <int D, int G>
 __device__ __forceinline__ uint32_t sim_kth(const uint32_t (&key)[D], int zeros, const SimGroup<G>& grp, uint32_t L,
-                                            uint32_t U, int below, int upto, int k) {
+                                            uint32_t U, int n, int k) {
     bool bisect = false;
+    int below = 0, upto = n;
     for (int it = 0; it < 80; ++it) {
         const bool live = L < U && upto - below > 1;
         if (!__any_sync(0xffffffffu, live)) break;
@@ -347,24 +378,68 @@ __device__ __forceinline__ uint32_t sim_kth(const uint32_t (&key)[D], int zeros,
     return L == U ? L : f;
 }
 
+// Median of the NPX pixels whose keys lie at `scratch` (KP words apart, 0 for a left-out
+// one), in every lane of the pixel's LP lanes: NaN if none is valid.
+template <class S>
+__device__ __forceinline__ float sim_median(const uint32_t* scratch, int lane, float fm) {
+    constexpr int LP = S::LP, KL = S::KL;
+    const uint32_t* mine = scratch + lane / LP * S::KP + lane % LP;
+    const SimGroup<LP> grp(lane);
+    uint32_t key[KL];
+    uint32_t kmin = 0xffffffffu, kmax = 0;
+    int cnt = 0;
+#pragma unroll
+    for (int i = 0; i < KL; ++i) {
+        key[i] = (i + 1) * LP <= S::K || i * LP + lane % LP < S::K ? mine[i * LP] : 0u;
+        cnt += key[i] ? 1 : 0;
+        kmin = ::min(kmin, key[i] - 1u);  // a left-out key wraps to the largest
+        kmax = ::max(kmax, key[i]);
+    }
+    const int n = grp.sum(cnt);
+    kmax = grp.max(kmax);
+    kmin = grp.min(kmin) + 1u;
+    const int k = n > 0 ? (n - 1) / 2 : 0;  // the median, or the lower one for even n
+    const uint32_t lo = sim_kth<KL, LP>(key, KL - cnt, grp, kmin, kmax, n, k);
+    // upper median: lo again if more than k + 1 keys are <= lo, else the smallest key above lo
+    int le = sim_count_below<KL>(key, lo + 1u) + cnt - KL;
+    uint32_t gt = 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < KL; ++i) gt = ::min(gt, key[i] > lo ? key[i] : 0xffffffffu);
+    le = grp.sum(le);
+    gt = grp.min(gt);
+    float res = __int_as_float(0x7fffffff);
+    if (n > 0) {
+        res = sim_unkey(lo) / fm;
+        if (!(n & 1)) {
+            const float up = sim_unkey(le >= k + 2 ? lo : gt) / fm;
+            res = (float)(((double)res + (double)up) * 0.5);
+        }
+    }
+    return res;
+}
+
 template <int H>
-__global__ void __launch_bounds__(SimShape<H>::THREADS, 512 / SimShape<H>::THREADS) k_similarity(SimArgs a) {
+__global__ void __launch_bounds__(SimShape<H>::THREADS, 1) k_similarity(SimArgs a) {
     using S = SimShape<H>;
-    constexpr int D = S::D, G = S::G, P = S::P;
+    constexpr int D = S::D, G = S::G, P = S::P, J = S::J;
     extern __shared__ __align__(16) unsigned char smem[];
     float2* stages = reinterpret_cast<float2*>(smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gl = lane % G;  // column offset dc = gl - H
+    const int gl = lane % G;  // column offset of pixel column j: dc = gl - H - j
     const int unit = warp * S::GPW + lane / G;
-    const int cu = unit % S::TC, rb = unit / S::TC;
-    const bool active = gl < D;
-    const int lc = active ? gl : D - 1;  // idle lanes read an in-bounds column
-    const int dc = gl - H;
-    const int hc = active ? a.hc[gl] : -1;
-    uint32_t run = 0;  // bit i: row offset i - H belongs to this lane's column of the circle
+    const int cu = unit % S::UC * J, rb = unit / S::UC;
+    const int lc = min(gl, D + J - 2);  // idle lanes read an in-bounds column
+    uint32_t run[J];  // bit i: row offset i - H belongs to this lane's column of pixel column j's circle
+    int slot[J];      // the circle's slot that row offset -H would have in that column
 #pragma unroll
-    for (int i = 0; i < 2 * H + 1; ++i)
-        if (i - H >= -hc && i - H <= hc && !(dc == 0 && i == H)) run |= 1u << i;
+    for (int j = 0; j < J; ++j) {
+        const int hc = gl >= j && gl - j < D ? a.hc[gl - j] : -1;
+        run[j] = 0;
+        slot[j] = hc >= 0 ? a.base[gl - j] - (H - hc) : 0;
+#pragma unroll
+        for (int i = 0; i < 2 * H + 1; ++i)
+            if (i - H >= -hc && i - H <= hc && !(gl - j == H && i == H)) run[j] |= 1u << i;
+    }
     const int64_t npix = (int64_t)a.rows * a.cols;
     const int nch = (a.m + kSimChunk - 1) / kSimChunk;
     const int my_tiles = a.tiles > (int)blockIdx.x ? (a.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -391,11 +466,16 @@ __global__ void __launch_bounds__(SimShape<H>::THREADS, 512 / SimShape<H>::THREA
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 
-    float acc[P][D];
+    float acc[J][P][D];
+    auto clear = [&]() {
 #pragma unroll
-    for (int p = 0; p < P; ++p)
+        for (int j = 0; j < J; ++j)
 #pragma unroll
-        for (int i = 0; i < D; ++i) acc[p][i] = 0.f;
+            for (int p = 0; p < P; ++p)
+#pragma unroll
+                for (int i = 0; i < D; ++i) acc[j][p][i] = 0.f;
+    };
+    clear();
     if (steps > 0) issue(0);
     for (int s = 0; s < steps; ++s) {
         if (s + 1 < steps) {
@@ -408,89 +488,90 @@ __global__ void __launch_bounds__(SimShape<H>::THREADS, 512 / SimShape<H>::THREA
         const int ch = s % nch;
         const float2* T = stages + (s & 1) * S::STAGE;
         const int nl = min(kSimChunk, a.m - ch * kSimChunk);
-        constexpr int kUnroll = H <= 7 ? 2 : 1;  // two layers in flight where registers allow
-#pragma unroll(kUnroll)
-        for (int j = 0; j < nl; ++j) {
-            const float2* colp = T + j * S::LAYER + (rb * P) * S::SW + cu + lc;
-            const float2* ownp = T + j * S::LAYER + (rb * P + H) * S::SW + cu + H;
-            float2 own[P], v[D + P - 1];
+#pragma unroll 1
+        for (int l = 0; l < nl; ++l) {
+            const float2* colp = T + l * S::LAYER + (rb * P) * S::SW + cu + lc;
+            const float2* ownp = T + l * S::LAYER + (rb * P + H) * S::SW + cu + H;
+            float2 own[J][P];
 #pragma unroll
-            for (int p = 0; p < P; ++p) own[p] = ownp[p * S::SW];
+            for (int p = 0; p < P; ++p)
 #pragma unroll
-            for (int t = 0; t < D + P - 1; ++t) v[t] = colp[t * S::SW];
-            // all real-part products first, then the imaginary ones: the two multiply-adds
-            // of an accumulator are far apart in the instruction stream
+                for (int j = 0; j < J; ++j) own[j][p] = ownp[p * S::SW + j];
 #pragma unroll
-            for (int t = 0; t < D + P - 1; ++t)
+            for (int t = 0; t < D + P - 1; ++t) {
+                const float2 v = colp[t * S::SW];
 #pragma unroll
                 for (int p = 0; p < P; ++p)
-                    if (t - p >= 0 && t - p < D) acc[p][t - p] = fmaf(own[p].x, v[t].x, acc[p][t - p]);
 #pragma unroll
-            for (int t = 0; t < D + P - 1; ++t)
+                    for (int j = 0; j < J; ++j)
+                        if (t - p >= 0 && t - p < D) acc[j][p][t - p] = fmaf(own[j][p].x, v.x, acc[j][p][t - p]);
 #pragma unroll
                 for (int p = 0; p < P; ++p)
-                    if (t - p >= 0 && t - p < D) acc[p][t - p] = fmaf(own[p].y, v[t].y, acc[p][t - p]);
+#pragma unroll
+                    for (int j = 0; j < J; ++j)
+                        if (t - p >= 0 && t - p < D) acc[j][p][t - p] = fmaf(own[j][p].y, v.y, acc[j][p][t - p]);
+            }
         }
         if (ch == nch - 1) {
-            // the tile's sums are complete: summaries of the group's P pixels, all lanes
-            // of the warp in step
+            // the tile's sums are complete: summaries of the group's pixels, all lanes of the
+            // warp in step
             const int tile = blockIdx.x + (s / nch) * gridDim.x;
-            const int r0 = (tile / a.tiles_c) * S::TR, c = (tile % a.tiles_c) * S::TC + cu;
+            const int r0 = (tile / a.tiles_c) * S::TR, tc0 = (tile % a.tiles_c) * S::TC, c = tc0 + cu;
             const float fm = (float)a.m;
-            const bool col_self = dc == 0 || (dc < 0 && c == 0) || (dc > 0 && c == a.cols - 1);
             const SimGroup<G> grp(lane);
+            // this warp's part of the stage just read
+            uint32_t* scratch = reinterpret_cast<uint32_t*>(stages + (s & 1) * S::STAGE) + warp * S::NPX * S::KP;
+            if (a.kind == 0) __syncthreads();  // every warp has read the stage
 #pragma unroll
             for (int p = 0; p < P; ++p) {
                 const int r = r0 + rb * P + p;
-                const bool inside = r < a.rows && c < a.cols;
-                // the pixel itself, reached through a clipped offset at the image edge
-                uint32_t self = 0;
-                if (col_self) {
-                    self = 1u << H;
-                    if (r == 0) self |= (1u << H) - 1u;
-                    if (r == a.rows - 1) self |= ((1u << D) - 1u) & ~((2u << H) - 1u);
-                }
-                const uint32_t vm = inside ? run & ~self : 0u;
-                uint32_t key[D];  // 0: left out
-                uint32_t kmin = 0xffffffffu, kmax = 0;
-                int cnt = 0;
 #pragma unroll
-                for (int i = 0; i < D; ++i) {
-                    const bool use = ((vm >> i) & 1u) && !isnan(acc[p][i]);
-                    key[i] = use ? sim_key(acc[p][i]) : 0u;
-                    cnt += use ? 1 : 0;
-                    kmin = ::min(kmin, use ? key[i] : 0xffffffffu);
-                    kmax = ::max(kmax, key[i]);
-                }
-                const int n = grp.sum(cnt);
-                const uint32_t gmax = grp.max(kmax);
-                float res = __int_as_float(0x7fffffff);
-                if (a.kind == 1) {
-                    if (n > 0) res = sim_unkey(gmax) / fm;
-                } else {
-                    const uint32_t gmin = grp.min(kmin);
-                    const int k = n > 0 ? (n - 1) / 2 : 0;  // the median, or the lower one for even n
-                    const uint32_t lo = sim_kth<D, G>(key, D - cnt, grp, gmin, gmax, 0, n, k);
-                    // upper median: lo again if more than k + 1 keys are <= lo, else the
-                    // smallest key above lo
-                    int le = sim_count_below<D>(key, lo + 1u) + cnt - D;
-                    uint32_t gt = 0xffffffffu;
+                for (int j = 0; j < J; ++j) {
+                    const int dc = gl - H - j;
+                    const bool inside = r < a.rows && c + j < a.cols;
+                    // the pixel itself, reached through a clipped offset at the image edge
+                    uint32_t self = 0;
+                    if (dc == 0 || (dc < 0 && c + j == 0) || (dc > 0 && c + j == a.cols - 1)) {
+                        self = 1u << H;
+                        if (r == 0) self |= (1u << H) - 1u;
+                        if (r == a.rows - 1) self |= ((1u << D) - 1u) & ~((2u << H) - 1u);
+                    }
+                    const uint32_t vm = inside ? run[j] & ~self : 0u;
+                    if (a.kind == 0) {
+                        // pixel of the warp's batch, slot of row offset -H in this lane's column
+                        uint32_t* dst = scratch + ((lane / G * S::PB + p % S::PB) * J + j) * S::KP + slot[j];
 #pragma unroll
-                    for (int i = 0; i < D; ++i) gt = ::min(gt, key[i] > lo ? key[i] : 0xffffffffu);
-                    le = grp.sum(le);
-                    gt = grp.min(gt);
-                    if (n > 0) {
-                        res = sim_unkey(lo) / fm;
-                        if (!(n & 1)) {
-                            const float up = sim_unkey(le >= k + 2 ? lo : gt) / fm;
-                            res = (float)(((double)res + (double)up) * 0.5);
+                        for (int i = 0; i < D; ++i) {
+                            const float v = acc[j][p][i];
+                            const uint32_t key = ((vm >> i) & 1u) && !isnan(v) ? sim_key(v) : 0u;
+                            if ((run[j] >> i) & 1u) dst[i > H && dc == 0 ? i - 1 : i] = key;
+                        }
+                    } else {
+                        uint32_t kmax = 0;
+#pragma unroll
+                        for (int i = 0; i < D; ++i) {
+                            const float v = acc[j][p][i];
+                            if (((vm >> i) & 1u) && !isnan(v)) kmax = ::max(kmax, sim_key(v));
+                        }
+                        kmax = grp.max(kmax);
+                        if (gl == 0 && inside) {
+                            const float none = __int_as_float(0x7fffffff);
+                            a.out[(int64_t)r * a.cols + c + j] = kmax ? sim_unkey(kmax) / fm : none;
                         }
                     }
                 }
-                if (gl == 0 && inside) a.out[(int64_t)r * a.cols + c] = res;
-#pragma unroll
-                for (int i = 0; i < D; ++i) acc[p][i] = 0.f;  // next tile
+                if (a.kind == 0 && p % S::PB == S::PB - 1) {
+                    __syncwarp();
+                    const float res = sim_median<S>(scratch, lane, fm);
+                    // pixel px of the batch: unit px / (PB J) of the warp, row p % PB, column j
+                    const int px = lane / S::LP, u2 = warp * S::GPW + px / (S::PB * J);
+                    const int rr = r0 + u2 / S::UC * P + p - (S::PB - 1) + px / J % S::PB;
+                    const int cc = tc0 + u2 % S::UC * J + px % J;
+                    if (lane % S::LP == 0 && rr < a.rows && cc < a.cols) a.out[(int64_t)rr * a.cols + cc] = res;
+                    __syncwarp();  // the scratch is written again
+                }
             }
+            clear();  // next tile
         }
         __syncthreads();  // the buffer just read is refilled by the next issue
     }
@@ -584,10 +665,9 @@ extern "C" dpl_status dpl_similarity(const float* unit, int64_t nlayers, int64_t
         return fail(DPL_ERR_INVALID_ARGUMENT, "dpl_similarity: complex arrays must be 8-byte aligned");
     const int H = search_radius - 1;
     SimArgs a{};
-    int K = 0, base[2 * kSimHMax + 1];
-    if (H > 0 && !circle_columns(search_radius, H, a.hc, base, &K))
+    if (H > 0 && (!circle_columns(search_radius, H, a.hc, a.base, &a.K) || a.K != kSimCircle[H]))
         return fail(DPL_ERR_UNSUPPORTED, "dpl_similarity: search circle has a non-contiguous column");
-    if (K == 0 || nlayers == 0) {
+    if (a.K == 0 || nlayers == 0) {
         // no offsets, or no layers (every pixel invalid): all NaN
         DPL_CUDA_TRY(cudaMemsetAsync(out, 0xff, (size_t)npix * sizeof(float), (cudaStream_t)stream));
         return DPL_OK;
