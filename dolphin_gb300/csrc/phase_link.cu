@@ -660,7 +660,7 @@ static dpl_status launch_pixel(PixArgs& a, cudaStream_t s, int* fb = nullptr, in
 // shape does not fit (then the plain SIMT form is used).
 // Shared-memory carve of the covariance kernel for nst operand stages, sized for up to
 // n SLCs, kpad region samples and npass passes (a batch carves once for all its items).
-static void tc_carve(TcArgs& a, int nst, int n, int kpad, int npass, bool tf32) {
+static void tc_carve(TcArgs& a, int nst, int n, int kpad, int kwords, int npass, bool tf32) {
     size_t o = 0;
     auto take = [&](size_t bytes, size_t al) {
         o = align_up(o, al);
@@ -672,7 +672,7 @@ static void tc_carve(TcArgs& a, int nst, int n, int kpad, int npass, bool tf32) 
     a.off_stage = take((size_t)nst * (tf32 ? kTcStageBytesTf : kTcStageBytes), 1024);
     a.z_bytes = (int)align_up((size_t)kTcKC * n * sizeof(cfloat), 16);
     a.off_z = take(kTcZBuf * (size_t)a.z_bytes, 16);
-    a.off_pbits = take((size_t)kTcN * (kpad / 32) * sizeof(uint32_t), 16);
+    a.off_pbits = take((size_t)kTcN * kwords * sizeof(uint32_t), 16);
     a.off_soff = take((size_t)kpad * sizeof(int), 16);
     a.off_runs = take((size_t)(kpad / kTcKC) * kTcRuns * sizeof(int2), 16);
     a.off_rows = take((size_t)npass * kTcRows * sizeof(uint32_t), 16);
@@ -698,28 +698,31 @@ static bool tc_configure(TcArgs& a, int n, int rows, int cols, int hy, int hx, i
     a.region_r = (kTcTileR - 1) * sy + wy;
     a.region_c = (kTcTileC - 1) * sx + wx;
     a.kpad = (int)(ceil_div((int64_t)a.region_r * a.region_c, kTcKC) * kTcKC);
-    a.kwords = a.kpad / 32;
     const int O = n * (n - 1) / 2;
     // pass 0: the diagonal and kTcRows - n pairs; then kTcRows pairs per pass
     a.npass = 1 + ceil_div(std::max(0, O - (kTcRows - n)), kTcRows);
-    // three operand stages where they fit in shared memory, else two
+    // three operand stages where they fit in shared memory, else two; an odd number of
+    // words per pixel's mask bits (the pixels then fall into different banks) where it fits
     for (a.nst = kTcMaxStages; a.nst >= 2; --a.nst) {
-        tc_carve(a, a.nst, n, a.kpad, a.npass, tf32);
+        for (a.kwords = (a.kpad / 32) | 1; a.kwords >= a.kpad / 32; --a.kwords) {
+            tc_carve(a, a.nst, n, a.kpad, a.kwords, a.npass, tf32);
+            if (a.smem_bytes <= 227 * 1024) break;
+        }
         if (a.smem_bytes <= 227 * 1024) break;
     }
-    return a.nst >= 2 && a.smem_bytes <= 227 * 1024;
+    // the tile rows' mask bits pass through the operand stages
+    const size_t raw = (size_t)kTcTileR * ((kTcTileC * wy * wx + 31) / 32 + 2) * sizeof(uint32_t);
+    return a.nst >= 2 && a.smem_bytes <= 227 * 1024 && raw <= 2 * (size_t)kTcStageBytes;
 }
 
 static dpl_status launch_cov_tc(int n, int rows, int cols, int hy, int hx, int sy, int sx, const cfloat* zt,
-                                const uint32_t* bits, int wpr, const uint8_t* nb_u8, float* Cg, int32_t* counts,
+                                const uint8_t* nb_u8, float* Cg, int32_t* counts,
                                 int* status, cudaStream_t s, bool tf32 = false) {
     TcArgs a{};
     if (!tc_configure(a, n, rows, cols, hy, hx, sy, sx, tf32))
         return fail(DPL_ERR_UNSUPPORTED, "tensor-core covariance: unsupported shape");
     if (a.out_rows == 0 || a.out_cols == 0) return DPL_OK;
     a.zt = zt;
-    a.bits = bits;
-    a.wpr = wpr;
     a.nb_u8 = nb_u8;
     a.Cg = Cg;
     a.counts = counts;
@@ -753,15 +756,16 @@ static dpl_status launch_cov_tc_batch(std::vector<TcArgs> items, bool tf32, int*
     if (items.empty()) return DPL_OK;
     if (items.size() > (size_t)kTcMaxItems) return fail(DPL_ERR_UNSUPPORTED, "batch: more than 16 stacks");
     std::stable_sort(items.begin(), items.end(), [](const TcArgs& x, const TcArgs& y) { return x.n > y.n; });
-    int nst = kTcMaxStages, nmax = 0, kpad = 0, npass = 0;
+    int nst = kTcMaxStages, nmax = 0, kpad = 0, kwords = 0, npass = 0;
     for (const TcArgs& t : items) {
+        kwords = std::max(kwords, t.kwords);
         nst = std::min(nst, t.nst);
         nmax = std::max(nmax, t.n);
         kpad = std::max(kpad, t.kpad);
         npass = std::max(npass, t.npass);
     }
     TcArgs carve{};
-    tc_carve(carve, nst, nmax, kpad, npass, tf32);
+    tc_carve(carve, nst, nmax, kpad, kwords, npass, tf32);
     if (carve.smem_bytes > 227 * 1024) return fail(DPL_ERR_UNSUPPORTED, "batch: covariance shared memory exceeds the SM limit");
     TcBatch b{};
     b.nitems = (int)items.size();
@@ -967,8 +971,6 @@ static dpl_status pl_begin(const dpl_pl_params* prm, const dpl_pl_inputs* in, co
                 tc_configure(S.tc, n, (int)P.rows, (int)P.cols, P.hy, P.hx, P.sy, P.sx, S.tf32);
     if (S.tc_fits) {
         S.tc.zt = w.zt;
-        S.tc.bits = nullptr;
-        S.tc.wpr = 0;
         S.tc.nb_u8 = in->neighbors;
         S.tc.Cg = w.Cg;
         S.tc.counts = a.counts;
@@ -993,7 +995,7 @@ static dpl_status pl_finish(PlState& S, cudaStream_t s, bool cov_done) {
         // chosen form: tensor-core covariance, then the solver on the planar matrices
         if (!cov_done) {
             st = timed(s, 0, [&] {
-                return launch_cov_tc(n, (int)P.rows, (int)P.cols, P.hy, P.hx, P.sy, P.sx, w.zt, nullptr, 0,
+                return launch_cov_tc(n, (int)P.rows, (int)P.cols, P.hy, P.hx, P.sy, P.sx, w.zt,
                                      S.in->neighbors, w.Cg, a.counts, w.status, s, S.tf32);
             });
             if (st != DPL_OK) return st;
@@ -1274,7 +1276,7 @@ extern "C" dpl_status dpl_covariance(const float* slc, int64_t nslc, int64_t row
     if (cov_form == 1 || !tc_configure(tcfit, n, (int)rows, (int)cols, hy, hx, sy, sx, cov_form == 3))
         return launch_pixel<kCovOnly>(a, s);
     DPL_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
-    st = launch_cov_tc(n, (int)rows, (int)cols, hy, hx, sy, sx, zt, nullptr, 0, neighbors, Cg, nullptr, status, s,
+    st = launch_cov_tc(n, (int)rows, (int)cols, hy, hx, sy, sx, zt, neighbors, Cg, nullptr, status, s,
                        cov_form == 3);
     if (st != DPL_OK) return st;
     const int64_t tot = a.npix * n * n;
