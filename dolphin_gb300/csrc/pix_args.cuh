@@ -20,7 +20,7 @@ struct PixLayout {
 };
 
 // C (packed complex) | G (n x ldg real) | S: staging for the covariance's window rows,
-// or R (packed complex), or the full n x n LU of the LU pass | v | d | piv
+// or R (packed complex), or the full n x n LU of the LU pass and its inverse | v | d | piv
 inline PixLayout make_layout(int n, int wx, bool lu) {
     PixLayout L{};
     const size_t T = (size_t)n * (n + 1) / 2;
@@ -37,7 +37,7 @@ inline PixLayout make_layout(int n, int wx, bool lu) {
     L.off_C = take(T * sizeof(cfloat));
     L.off_G = take((size_t)n * L.ldg * sizeof(float));
     size_t s_bytes = std::max((size_t)L.stg * sizeof(cfloat), T * sizeof(cfloat));
-    if (lu) s_bytes = std::max(s_bytes, (size_t)n * n * sizeof(cfloat));
+    if (lu) s_bytes = std::max(s_bytes, (size_t)n * (n + (n | 1)) * sizeof(cfloat));  // LU, explicit inverse
     L.off_S = take(s_bytes);
     L.off_v = take(64 * sizeof(cfloat));
     L.off_d = take(64 * sizeof(float));

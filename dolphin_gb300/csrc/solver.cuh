@@ -264,6 +264,71 @@ __device__ void s_lu_solve(const cfloat* A, int n, const int* src, cfloat (&x)[N
     for (int q = 0; q < NB; ++q) x[q] = w[q];
 }
 
+template <int NB>
+__device__ void s_publish(cfloat* vpub, const cfloat (&x)[NB], int n, int lane) {
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NB; ++q)
+        if (lane + 32 * q < n) vpub[lane + 32 * q] = x[q];
+    __syncwarp();
+}
+
+// Whether inverse iteration with this factorisation is far from its stopping rule after
+// all its steps: the same iteration with the explicit inverse M (n x (n | 1), one column
+// per lane), whose steps are a product instead of 2 n dependent ones with n divisions.
+// True only if no step came within ten times the rule; a NaN difference gives false.
+template <int NB>
+__device__ bool s_lu_stalls(const cfloat* A, int n, const int* src, cfloat* M, cfloat* vpub, int lane) {
+    const int ld = n | 1;
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int j = lane + 32 * q;
+        if (j < n) {
+            cfloat* col = M + j;
+            for (int i = 0; i < n; ++i) {
+                cfloat acc = cmake(src[i] == j ? 1.f : 0.f, 0.f);
+#pragma unroll 4
+                for (int k = 0; k < i; ++k) acc = csub(acc, cmul(A[i * n + k], col[k * ld]));
+                col[i * ld] = acc;
+            }
+            for (int i = n - 1; i >= 0; --i) {
+                cfloat acc = col[i * ld];
+#pragma unroll 4
+                for (int k = i + 1; k < n; ++k) acc = csub(acc, cmul(A[i * n + k], col[k * ld]));
+                const cfloat d = A[i * n + i];
+                col[i * ld] = cscale(cmulc(acc, d), 1.f / cabs2(d));
+            }
+        }
+    }
+    cfloat v[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) v[q] = lane + 32 * q < n ? cmake(rsqrtf((float)n), 0.f) : cmake(0.f, 0.f);
+    for (int it = 1; it < 50; ++it) {
+        s_publish<NB>(vpub, v, n, lane);
+        cfloat x[NB];
+        float n2 = 0.f, dd = 0.f;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const int i = lane + 32 * q;
+            x[q] = cmake(0.f, 0.f);
+            if (i < n) {
+#pragma unroll 4
+                for (int k = 0; k < n; ++k) x[q] = cfma(x[q], M[i * ld + k], vpub[k]);
+            }
+            n2 += cabs2(x[q]);
+        }
+        const float inv = rsqrtf(warp_sum(n2));
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            x[q] = cscale(x[q], inv);
+            dd += cabs2(csub(x[q], v[q]));
+            v[q] = x[q];
+        }
+        if (!(sqrtf(warp_sum(dd)) > 1e-4f)) return false;
+    }
+    return true;
+}
+
 // |c| by the approximate square root (relative error below 2^-22)
 __device__ __forceinline__ float s_abs_approx(cfloat c) {
     float g;
@@ -293,15 +358,6 @@ __device__ void s_hermv(const cfloat* H, int n, const cfloat* vpub, cfloat (&y)[
         }
         y[q] = acc;
     }
-}
-
-template <int NB>
-__device__ void s_publish(cfloat* vpub, const cfloat (&x)[NB], int n, int lane) {
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < NB; ++q)
-        if (lane + 32 * q < n) vpub[lane + 32 * q] = x[q];
-    __syncwarp();
 }
 
 // Normalising iteration x <- op(v) / |op(v)| until |x - v| <= 1e-5 or 49 steps; true
@@ -424,7 +480,13 @@ __device__ void solve_pixel(const PixArgs& a, int64_t p, const SolveMats& m, int
                 }
             }
             __syncwarp();
-            converged = s_iterate<NB>(v, [&](cfloat(&x)[NB]) { s_lu_solve<NB>(A, n, src, x, lane); });
+            // a pixel that the dense eigensolver takes over needs no iterate: most listed
+            // pixels use all 49 steps, 1.4 M of the pass's 1.65 M cycles at N = 30 (the pass
+            // on 1034 x 1046 pixels: 806 -> 353 us; at N = 10 on 128 x 128: 156 -> 60 us)
+            if (a.nc_list && s_lu_stalls<NB>(A, n, src, A + n * n, m.v, lane))
+                converged = false;
+            else
+                converged = s_iterate<NB>(v, [&](cfloat(&x)[NB]) { s_lu_solve<NB>(A, n, src, x, lane); });
             s_publish<NB>(m.v, v, n, lane);
             float s = 0.f;
 #pragma unroll
