@@ -13,7 +13,8 @@
 // warp_covariance, so that both give the same sums bit for bit).  A thread per matrix row
 // over all 32 columns, as in warp_covariance, computes 1024 products per sample where
 // N = 21 needs 231; the blocks compute 252.  512 x 384 outputs, 11 x 23 windows, N = 21:
-// 4.0 ms, 18.7 T operations/s, half of what the pipe issues.
+// 3.6 ms, 21 T operations/s, 57 % of what the pipe issues (a fully set window row skips the
+// search for set bits and takes two samples per turn: 4.0 ms without).
 //
 // Output: planar per pixel and normalised, Cg[p][0 .. N^2): diagonal, then (Re, Im) per
 // lower pair, C_ij = numer_ij / sqrt(amp_i amp_j) where that root is > 1e-6, else 0
@@ -27,13 +28,14 @@ constexpr int kCovSimtPad = 16;  // elements behind a staged row that a last blo
 inline int cov_simt_block(int n) { return n <= 49 ? (n + 6) / 7 : (n + 9) / 10; }
 
 template <int B>
-__global__ void __launch_bounds__(256) k_cov_simt(const PixArgs a, float* __restrict__ Cg, int row_elems) {
+__global__ void __launch_bounds__(256, B <= 3 ? 3 : B <= 5 ? 2 : 1) k_cov_simt(const PixArgs a, float* __restrict__ Cg, int row_elems) {
     extern __shared__ __align__(16) unsigned char cov_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     cfloat* buf = reinterpret_cast<cfloat*>(cov_smem) + (size_t)warp * 2 * row_elems;
     const int n = a.n, wy = 2 * a.hy + 1, wx = 2 * a.hx + 1;
     const int T = (n + B - 1) / B, nblocks = T * (T + 1) / 2;
     const int row_len = wx * n;
+    const uint64_t full_row = wx >= 64 ? ~0ull : (1ull << wx) - 1ull;
     for (int64_t p = (int64_t)blockIdx.x * nwarps + warp; p < a.npix; p += (int64_t)gridDim.x * nwarps) {
         const int out_r = (int)(p / a.out_cols), out_c = (int)(p - (int64_t)out_r * a.out_cols);
         const int r0 = clamp_start_i(a.sy / 2 + out_r * a.sy, a.hy, wy, a.rows);
@@ -76,27 +78,33 @@ __global__ void __launch_bounds__(256) k_cov_simt(const PixArgs a, float* __rest
                 const uint64_t rm = row_mask(a, p, wa, wx, lane);
                 count += __popcll(rm);
                 const cfloat* row = buf + (wa & 1) * row_elems;
-#pragma unroll 1
-                for (int half = 0; half < 2; ++half) {
-                    uint32_t m = (uint32_t)(rm >> (32 * half));
-#pragma unroll 1
-                    while (m) {
-                        const int b = __ffs(m) - 1 + 32 * half;
-                        m &= m - 1u;
-                        const cfloat* s = row + b * n;
-                        cfloat zi[B], zj[B];
+                auto add = [&](const cfloat* si, const cfloat* sj) {
+                    cfloat zi[B], zj[B];
 #pragma unroll
-                        for (int x = 0; x < B; ++x) {
-                            zi[x] = s[bi * B + x];
-                            zj[x] = s[bj * B + x];
+                    for (int x = 0; x < B; ++x) {
+                        zi[x] = si[x];
+                        zj[x] = sj[x];
+                    }
+#pragma unroll
+                    for (int x = 0; x < B; ++x)
+#pragma unroll
+                        for (int y = 0; y < B; ++y) {
+                            are[x][y] = fadd(are[x][y], fmaf(zi[x].re, zj[y].re, fmul(zi[x].im, zj[y].im)));
+                            aim[x][y] = fadd(aim[x][y], fmaf(zi[x].im, zj[y].re, -fmul(zi[x].re, zj[y].im)));
                         }
-#pragma unroll
-                        for (int x = 0; x < B; ++x)
-#pragma unroll
-                            for (int y = 0; y < B; ++y) {
-                                are[x][y] = fadd(are[x][y], fmaf(zi[x].re, zj[y].re, fmul(zi[x].im, zj[y].im)));
-                                aim[x][y] = fadd(aim[x][y], fmaf(zi[x].im, zj[y].re, -fmul(zi[x].re, zj[y].im)));
-                            }
+                };
+                const cfloat *si = row + bi * B, *sj = row + bj * B;
+                if (rm == full_row) {
+#pragma unroll(B <= 3 ? 2 : 1)
+                    for (int b = 0; b < wx; ++b, si += n, sj += n) add(si, sj);
+                } else {
+#pragma unroll 1
+                    for (int half = 0; half < 2; ++half) {
+#pragma unroll 1
+                        for (uint32_t m = (uint32_t)(rm >> (32 * half)); m; m &= m - 1u) {
+                            const int b = (__ffs(m) - 1 + 32 * half) * n;
+                            add(si + b, sj + b);
+                        }
                     }
                 }
                 __syncwarp();  // the row's buffer is refilled by the next stage

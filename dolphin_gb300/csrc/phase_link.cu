@@ -1010,8 +1010,8 @@ static dpl_status pl_finish(PlState& S, cudaStream_t s, bool cov_done) {
         // form.  Its explicit inverses cost accuracy where a pixel is ill-conditioned: those
         // few pixels, and the undecided ones (|Gamma| not positive definite), are listed and
         // solved by the plain form, then the LU pass takes what both listed.
-        // 512 x 384 outputs, strides 3 x 6, 11 x 23 window, N = 21: 21.1 -> 6.4 ms on the device
-        // (the fused k_pixel took 20.6 ms; k_cov_simt 4.0, k_solve_reg 1.5, the list 0.3).
+        // 512 x 384 outputs, strides 3 x 6, 11 x 23 window, N = 21: 21.1 -> 5.9 ms on the device
+        // (the fused k_pixel took 20.6 ms; k_cov_simt 3.6, k_solve_reg 1.5, the list 0.3).
         st = timed(s, 0, [&] { return launch_cov_simt<1>(cov_simt_block(n), a, w.Cg, s); });
         if (st != DPL_OK) return st;
         st = timed(s, 1, [&]() -> dpl_status {
