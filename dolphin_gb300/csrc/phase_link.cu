@@ -41,44 +41,56 @@ __device__ __forceinline__ int clamp_start_i(int center, int half, int size, int
 // k_prep
 // ---------------------------------------------------------------------------------
 constexpr int kPrepPix = 64;
+inline size_t prep_smem(int n) { return (size_t)kPrepPix * (n | 1) * sizeof(cfloat); }
 
+// HBM-bound by its bytes (8 N in, 8 N + 5 out per pixel).  A tile of 64 pixels is
+// transposed through shared memory at an odd pitch (conflict-free both ways); NaNs and the
+// per-SLC "has a sample" bits are found in the loading loop, where a warp holds one SLC's
+// samples, and only a wanted amplitude mean walks the dates of a pixel.  (The walk for
+// every pixel, by a quarter of the threads and with the magnitudes: 1034 x 1046 pixels at
+// N = 30, 188 us, 123 us now; 1536 x 2304 at N = 21, 445 us, 295 us now.)
 __global__ void __launch_bounds__(256) k_prep(const cfloat* __restrict__ slc, int n, int64_t npix,
                                               const uint8_t* __restrict__ nodata_in,
                                               const uint8_t* __restrict__ ps_in, int mask_input_ps,
                                               int nan_is_nodata, uint8_t* __restrict__ flags,
                                               cfloat* __restrict__ zt,
                                               float* __restrict__ avgmag, unsigned int* __restrict__ valid_bits) {
-    extern __shared__ cfloat prep_s[];  // [kPrepPix][n + 1]
+    extern __shared__ cfloat prep_s[];  // [kPrepPix][n | 1]
     __shared__ uint8_t ign[kPrepPix];
-    __shared__ unsigned long long vbits;
-    const int ld = n + 1;
+    __shared__ unsigned int nan_px[kPrepPix / 32];  // bit px: some sample is NaN
+    __shared__ unsigned int vbits[2];
+    const int ld = n | 1;
     const int64_t p0 = (int64_t)blockIdx.x * kPrepPix;
-    if (threadIdx.x == 0) vbits = 0ull;
-    for (int i = threadIdx.x; i < n * kPrepPix; i += blockDim.x) {
-        const int t = i / kPrepPix, px = i - t * kPrepPix;
+    if (threadIdx.x < kPrepPix / 32) nan_px[threadIdx.x] = 0u;
+    if (threadIdx.x < 2) vbits[threadIdx.x] = 0u;
+    __syncthreads();
+    {
+        // a warp takes 32 pixels of every fourth SLC
+        const int px = threadIdx.x % kPrepPix, half = px >> 5;
         const int64_t p = p0 + px;
-        prep_s[px * ld + t] = p < npix ? slc[(int64_t)t * npix + p] : cmake(0.f, 0.f);
+        const bool in = p < npix;
+        const cfloat* src = slc + (in ? p : 0);
+        unsigned int nans = 0u, valid[2] = {0u, 0u};
+#pragma unroll 8
+        for (int t = threadIdx.x / kPrepPix; t < n; t += 256 / kPrepPix) {
+            const cfloat z = in ? src[(int64_t)t * npix] : cmake(0.f, 0.f);
+            const bool nan = cisnan(z);
+            nans |= __ballot_sync(0xffffffffu, nan);
+            if (__any_sync(0xffffffffu, in && !nan)) valid[t >> 5] |= 1u << (t & 31);
+            prep_s[px * ld + t] = z;
+        }
+        if ((threadIdx.x & 31) == 0) {
+            if (nans) atomicOr(&nan_px[half], nans);
+            if (valid[0]) atomicOr(&vbits[0], valid[0]);
+            if (valid[1]) atomicOr(&vbits[1], valid[1]);
+        }
     }
     __syncthreads();
     if (threadIdx.x < kPrepPix) {
         const int px = threadIdx.x;
         const int64_t p = p0 + px;
         if (p < npix) {
-            bool anynan = false;
-            unsigned long long vb = 0ull;
-            float msum = 0.f;
-            int mcnt = 0;
-            for (int t = 0; t < n; ++t) {
-                cfloat z = prep_s[px * ld + t];
-                bool nan = cisnan(z);
-                anynan |= nan;
-                if (!nan) {
-                    vb |= 1ull << t;
-                    float m = hypotf(z.re, z.im);
-                    msum = mcnt == 0 ? m : fadd(msum, m);
-                    ++mcnt;
-                }
-            }
+            const bool anynan = (nan_px[px >> 5] >> (px & 31)) & 1u;
             // run_phase_linking marks a pixel with any NaN as nodata (_core.py:181);
             // the bare covariance masks NaN samples one by one (covariance.py:122-123)
             const bool nodata = (nodata_in && nodata_in[p]) || (nan_is_nodata && anynan);
@@ -86,24 +98,41 @@ __global__ void __launch_bounds__(256) k_prep(const cfloat* __restrict__ slc, in
             const bool ignore = nodata || (mask_input_ps && ps);
             flags[p] = (nodata ? kNodata : 0) | (ps ? kPs : 0) | (ignore ? kIgnore : 0);
             ign[px] = ignore;
-            if (avgmag) avgmag[p] = fdiv(msum, (float)mcnt);
-            if (vb) atomicOr(&vbits, vb);
+            if (avgmag) {
+                float msum = 0.f;
+                int mcnt = 0;
+                for (int t = 0; t < n; ++t) {
+                    const cfloat z = prep_s[px * ld + t];
+                    if (!cisnan(z)) {
+                        const float m = hypotf(z.re, z.im);
+                        msum = mcnt == 0 ? m : fadd(msum, m);
+                        ++mcnt;
+                    }
+                }
+                avgmag[p] = fdiv(msum, (float)mcnt);
+            }
         } else {
             ign[px] = 1;
         }
+    } else if (threadIdx.x < kPrepPix + 2) {
+        const int w = threadIdx.x - kPrepPix;
+        if (vbits[w]) atomicOr(valid_bits + w, vbits[w]);
     }
     __syncthreads();
-    if (threadIdx.x == 0 && vbits) {
-        atomicOr(valid_bits, (unsigned int)(vbits & 0xffffffffull));
-        atomicOr(valid_bits + 1, (unsigned int)(vbits >> 32));
-    }
-    for (int i = threadIdx.x; i < kPrepPix * n; i += blockDim.x) {
-        const int px = i / n, t = i - px * n;
-        const int64_t p = p0 + px;
-        if (p < npix) {
-            cfloat z = prep_s[px * ld + t];
-            if (ign[px] || cisnan(z)) z = cmake(0.f, 0.f);
-            zt[p * n + t] = z;
+    // consecutive elements of the tile per thread: (px, t) advanced without a division
+    const int total = (int)(npix - p0 < kPrepPix ? npix - p0 : kPrepPix) * n;
+    const int dpx = 256 / n, dt = 256 - dpx * n;
+    int px = threadIdx.x / n, t = threadIdx.x - px * n;
+    cfloat* dst = zt + p0 * n;
+    for (int i = threadIdx.x; i < total; i += 256) {
+        cfloat z = prep_s[px * ld + t];
+        if (ign[px] || cisnan(z)) z = cmake(0.f, 0.f);
+        dst[i] = z;
+        px += dpx;
+        t += dt;
+        if (t >= n) {
+            t -= n;
+            ++px;
         }
     }
 }
@@ -430,36 +459,81 @@ struct PostArgs {
     int* status;
 };
 
+
+// HBM-bound by its bytes (12 N in, 12 N out per pixel).  A tile of kPostPix pixels'
+// eigenvectors and CRLBs comes in as the contiguous block it is and leaves by planes
+// through shared memory (odd pitch), 256 / kPostPix threads per pixel; kDirect: a thread
+// per pixel reads its own rows, as short as a sector or two.  The tile by depth, from
+// measurements at 64, 128 and 256 pixels (us, and a thread per pixel with direct reads):
+// N = 6, 700 x 700: 44, 31, 24 (18); N = 10, 522 x 522: 34, 21, 19 (20); N = 21, 512 x 512:
+// 43, 38, 42 (51); N = 30, 800 x 800: 114, 107, 159 (180); N = 45, 400 x 400: 43, 50, 108 (80).
+template <int kPostPix, bool kDirect>
 __global__ void __launch_bounds__(256) k_post(PostArgs a) {
+    extern __shared__ __align__(16) unsigned char post_s[];
+    __shared__ int s_br[kPostPix], s_bc[kPostPix];
+    __shared__ uint8_t s_kind[kPostPix];  // bit 0: all nodata, bit 1: some PS
+    const int ld = a.n | 1;
+    cfloat* sv = reinterpret_cast<cfloat*>(post_s);
+    float* sc = reinterpret_cast<float*>(sv + kPostPix * ld);
     const int64_t P = (int64_t)a.out_rows * a.out_cols;
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
-    const int orow = (int)(p / a.out_cols), ocol = (int)(p - (int64_t)orow * a.out_cols);
     const int64_t npix_in = (int64_t)a.rows * a.cols;
-    bool all_nodata = true, any_ps = false;
-    float best = -INFINITY;
-    int br = -1, bc = -1, nps = 0;
-    for (int dr = 0; dr < a.sy; ++dr) {
-        for (int dc = 0; dc < a.sx; ++dc) {
-            const int r = orow * a.sy + dr, c = ocol * a.sx + dc;
-            const uint8_t f = a.flags[(int64_t)r * a.cols + c];
-            all_nodata &= (f & kNodata) != 0;
-            if (f & kPs) {
-                any_ps = true;
-                ++nps;
-                const float mg = a.mag[(int64_t)r * a.cols + c];
-                if (!isnan(mg) && mg > best) {
-                    best = mg;
-                    br = r;
-                    bc = c;
-                }
+    const int64_t p0 = (int64_t)blockIdx.x * kPostPix;
+    const int count = (int)(P - p0 < kPostPix ? P - p0 : kPostPix);
+    if (!kDirect) {
+        const int total = count * a.n, dpx = 256 / a.n, dt = 256 - dpx * a.n;
+        int px = threadIdx.x / a.n, t = threadIdx.x - px * a.n;
+        for (int i = threadIdx.x; i < total; i += 256) {
+            sv[px * ld + t] = a.V[p0 * a.n + i];
+            sc[px * ld + t] = a.CR[p0 * a.n + i];
+            px += dpx;
+            t += dt;
+            if (t >= a.n) {
+                t -= a.n;
+                ++px;
             }
         }
     }
-    if (any_ps && a.use_max_ps && br < 0) atomicExch(a.status, (int)DPL_ERR_INVALID_ARGUMENT);
+    if ((int)threadIdx.x < count) {
+        const int64_t p = p0 + threadIdx.x;
+        const int orow = (int)(p / a.out_cols), ocol = (int)(p - (int64_t)orow * a.out_cols);
+        bool all_nodata = true, any_ps = false;
+        float best = -INFINITY;
+        int br = -1, bc = -1;
+        for (int dr = 0; dr < a.sy; ++dr) {
+            for (int dc = 0; dc < a.sx; ++dc) {
+                const int r = orow * a.sy + dr, c = ocol * a.sx + dc;
+                const uint8_t f = a.flags[(int64_t)r * a.cols + c];
+                all_nodata &= (f & kNodata) != 0;
+                if (f & kPs) {
+                    any_ps = true;
+                    const float mg = a.mag[(int64_t)r * a.cols + c];
+                    if (!isnan(mg) && mg > best) {
+                        best = mg;
+                        br = r;
+                        bc = c;
+                    }
+                }
+            }
+        }
+        if (any_ps && a.use_max_ps && br < 0) atomicExch(a.status, (int)DPL_ERR_INVALID_ARGUMENT);
+        s_br[threadIdx.x] = br;
+        s_bc[threadIdx.x] = bc;
+        s_kind[threadIdx.x] = (all_nodata ? 1 : 0) | (any_ps ? 2 : 0);
+        float tc = a.tcoh[p];
+        if (any_ps) tc = 1.f;
+        if (all_nodata) tc = nanf("");
+        a.tcoh[p] = tc;
+    }
+    __syncthreads();
+    const int px = threadIdx.x % kPostPix;
+    if (px >= count) return;
+    const int64_t p = p0 + px;
+    const bool all_nodata = s_kind[px] & 1, any_ps = s_kind[px] & 2;
+    const int br = s_br[px], bc = s_bc[px];
+    const int orow = (int)(p / a.out_cols), ocol = (int)(p - (int64_t)orow * a.out_cols);
     const int in_r = a.sy / 2 + orow * a.sy, in_c = a.sx / 2 + ocol * a.sx;
-    for (int t = 0; t < a.n; ++t) {
-        cfloat out = cphasor(a.V[p * a.n + t]);
+    for (int t = threadIdx.x / kPostPix; t < a.n; t += 256 / kPostPix) {
+        cfloat out = cphasor(kDirect ? a.V[p * a.n + t] : sv[px * ld + t]);
         if (any_ps) {
             const float amp = cabs(out);
             if (a.use_max_ps) {
@@ -493,12 +567,16 @@ __global__ void __launch_bounds__(256) k_post(PostArgs a) {
         }
         if (all_nodata) out = cmake(nanf(""), 0.f);
         a.cpx[(int64_t)t * P + p] = out;
-        a.crlb[(int64_t)t * P + p] = a.CR[p * a.n + t];
+        a.crlb[(int64_t)t * P + p] = kDirect ? a.CR[p * a.n + t] : sc[px * ld + t];
     }
-    float tc = a.tcoh[p];
-    if (any_ps) tc = 1.f;
-    if (all_nodata) tc = nanf("");
-    a.tcoh[p] = tc;
+}
+
+template <int kPostPix, bool kDirect>
+static dpl_status launch_post(const PostArgs& q, int64_t npix, cudaStream_t s) {
+    const size_t smem = kDirect ? 0 : (size_t)kPostPix * (q.n | 1) * (sizeof(cfloat) + sizeof(float));
+    DPL_CUDA_TRY(cudaFuncSetAttribute(k_post<kPostPix, kDirect>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_post<kPostPix, kDirect><<<ceil_div(npix, kPostPix), 256, smem, s>>>(q);
+    return check_launch("k_post");
 }
 
 // ---------------------------------------------------------------------------------
@@ -926,7 +1004,7 @@ static dpl_status pl_begin(const dpl_pl_params* prm, const dpl_pl_inputs* in, co
     S.Pout = (int64_t)S.out_rows * S.out_cols;
     DPL_CUDA_TRY(cudaMemsetAsync(w.status, 0, kPlStatusBytes, s));
     {
-        size_t smem = (size_t)kPrepPix * (n + 1) * sizeof(cfloat);
+        const size_t smem = prep_smem(n);
         DPL_CUDA_TRY(cudaFuncSetAttribute(k_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_prep<<<ceil_div(npix, kPrepPix), 256, smem, s>>>(
             reinterpret_cast<const cfloat*>(in->slc), n, npix, in->nodata_mask, in->ps_mask, P.mask_input_ps, 1, w.flags,
@@ -1063,8 +1141,10 @@ static dpl_status pl_finish(PlState& S, cudaStream_t s, bool cov_done) {
     q.tcoh = S.out->temp_coh;
     q.crlb = S.out->crlb_std_dev;
     q.status = w.status;
-    k_post<<<ceil_div(S.Pout, 256), 256, 0, s>>>(q);
-    return check_launch("k_post");
+    if (n <= 8) return launch_post<256, true>(q, S.Pout, s);
+    if (n <= 12) return launch_post<256, false>(q, S.Pout, s);
+    if (n <= 36) return launch_post<128, false>(q, S.Pout, s);
+    return launch_post<64, false>(q, S.Pout, s);
 }
 
 // Enqueues the whole pipeline on `stream` without synchronising.
@@ -1252,7 +1332,7 @@ extern "C" dpl_status dpl_covariance(const float* slc, int64_t nslc, int64_t row
     cfloat* zt = ws.take<cfloat>(rows * cols * nslc);
     float* Cg = ws.take<float>(rows * cols * nslc * nslc);
     const int64_t npix = rows * cols;
-    size_t smem = (size_t)kPrepPix * (n + 1) * sizeof(cfloat);
+    const size_t smem = prep_smem(n);
     DPL_CUDA_TRY(cudaFuncSetAttribute(k_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_prep<<<ceil_div(npix, kPrepPix), 256, smem, s>>>(reinterpret_cast<const cfloat*>(slc), n, npix, nullptr, nullptr,
                                                        0, 0, flags, zt, nullptr, vb);
