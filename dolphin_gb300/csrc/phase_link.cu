@@ -293,85 +293,98 @@ __global__ void __launch_bounds__(256) k_pixel(PixArgs a) {
 }
 
 // ---------------------------------------------------------------------------------
-// k_eigh: the dense eigensolver for the listed non-converged pixels (eigh.cuh), one
-// warp per pixel, a persistent grid over the list
+// k_eigh: the dense eigensolver for the listed non-converged pixels (eigh.cuh), W warps
+// per pixel, a persistent grid over the list
 // ---------------------------------------------------------------------------------
-__global__ void __launch_bounds__(32) k_eigh(PixArgs a, EighLayout L) {
-    extern __shared__ __align__(16) unsigned char eigh_smem[];
-    const int lane = threadIdx.x;
-    cfloat* C = reinterpret_cast<cfloat*>(eigh_smem + L.off_C);
-    cfloat* A = reinterpret_cast<cfloat*>(eigh_smem + L.off_A);
-    double* G = reinterpret_cast<double*>(eigh_smem + L.off_A);  // |Gamma| work matrix, until A is formed
-    double* col = reinterpret_cast<double*>(eigh_smem + L.off_col);
-    const EighVec V = eigh_vectors(eigh_smem, L);
-    cfloat* w = V.w;
+// the listed pixels idx, idx + stride, ... with the warps of t
+template <int W>
+__device__ __forceinline__ void eigh_pixels(const PixArgs& a, const EighLayout& L, unsigned char* smem, int idx,
+                                            int stride, int count, const EighCta<W>& t) {
+    if (idx >= count) return;
+    const int lane = t.lane;
     const int n = a.n, ld = L.ld, lag = a.baseline_lag;
-    const int count = *a.nc_count;
-    for (int idx = blockIdx.x; idx < count; idx += gridDim.x) {
+    cfloat* C = reinterpret_cast<cfloat*>(smem + L.off_C);
+    cfloat* A = reinterpret_cast<cfloat*>(smem + L.off_A);
+    double* G = reinterpret_cast<double*>(smem + L.off_A);  // |Gamma| work matrix, until A is formed
+    const EighVec V = eigh_vectors<W>(smem, L, n);
+    cfloat* w = V.u;
+    const int npairs = n * (n - 1) / 2, ntri = n * (n + 1) / 2;
+    for (int i = t.tid; i < n; i += t.T)
+        for (int j = 0; j <= i; ++j) V.tri[i * (i + 1) / 2 + j] = (unsigned short)(i << 8 | j);
+    for (; idx < count; idx += stride) {
         const int64_t p = a.nc_list[idx];
-        __syncwarp();
+        t.sync();
         // the coherence, normalised as the solvers read it
         if (a.Cplanar) {
             const float* src = a.Cplanar + p * n * n;
             float* rv = reinterpret_cast<float*>(w);
-            for (int i = lane; i < n; i += 32) rv[i] = __frsqrt_rn(src[i]);
-            __syncwarp();
-            for (int i = lane; i < n; i += 32) {
-                const float f = rv[i] * rv[i];
+            for (int i = t.tid; i < n; i += t.T) {
+                const float r = __frsqrt_rn(src[i]), f = r * r;
+                rv[i] = r;
                 C[i * ld + i] = cmake(f < 1e6f ? src[i] * f : 0.f, 0.f);
             }
-            // lower pairs (r, c), c < r, at e = r(r-1)/2 + c: every lane walks the pairs
-            // e = lane, lane + 32, ..., so its loads do not wait on one another
-            const int npairs = n * (n - 1) / 2;
-            int r = 1, c = lane;
-            while (c >= r) c -= r++;
-            for (int e = lane; e < npairs; e += 32) {
+            t.sync();
+            // lower pairs (r, c), c < r, at e = r(r-1)/2 + c
+#pragma unroll 4
+            for (int e = t.tid; e < npairs; e += t.T) {
+                const int r = (V.tri[e] >> 8) + 1, c = V.tri[e] & 255;
                 const float f = rv[r] * rv[c];
                 cfloat v = f < 1e6f ? cmake(src[n + 2 * e] * f, src[n + 2 * e + 1] * f) : cmake(0.f, 0.f);
                 if (lag > 0 && r - c >= lag) v = cmake(0.f, 0.f);
                 C[r * ld + c] = v;
                 C[c * ld + r] = cconj(v);
-                c += 32;
-                while (c >= r) c -= r++;
             }
         } else {
             const cfloat* src = a.Cin + p * n * n;
-            for (int r = 0; r < n; ++r)
-                for (int c = lane; c <= r; c += 32) {
-                    cfloat v = src[r * n + c];
-                    if (lag > 0 && r - c >= lag) v = cmake(0.f, 0.f);
-                    C[r * ld + c] = v;
-                    C[c * ld + r] = cconj(v);
-                }
+#pragma unroll 4
+            for (int e = t.tid; e < ntri; e += t.T) {
+                const int r = V.tri[e] >> 8, c = V.tri[e] & 255;
+                cfloat v = src[r * n + c];
+                if (lag > 0 && r - c >= lag) v = cmake(0.f, 0.f);
+                C[r * ld + c] = v;
+                C[c * ld + r] = cconj(v);
+            }
         }
-        __syncwarp();
+        t.sync();
         const bool evd = a.est[p] == 0;  // the estimator the solver chose
         bool ok = true;
         if (!evd) {
             // |Gamma| + 1e-6 I inverted in double; A = |Gamma|^{-1} o C (lower triangles)
-            for (int i = 0; i < n; ++i)
-                for (int j = lane; j <= i; j += 32)
-                    G[i * ld + j] = (double)s_gamma(a, C[i * ld + j], i == j) + (i == j ? 1e-6 : 0.0);
-            ok = e_inverse_spd(G, ld, col, col + kEighMaxN, n, lane);
-            if (ok)  // in place: each element of G is read, then A written over it, by one lane
-                for (int i = 0; i < n; ++i)
-                    for (int j = lane; j <= i; j += 32) {
-                        const float gi = (float)G[i * ld + j];
-                        A[i * ld + j] = cscale(C[i * ld + j], gi);
-                    }
-        } else {
-            for (int i = 0; i < n; ++i)
-                for (int j = lane; j <= i; j += 32) {
-                    const cfloat c = C[i * ld + j];
-                    A[i * ld + j] = cscale(c, sqrtf(c.re * c.re + c.im * c.im));
+            for (int e = t.tid; e < ntri; e += t.T) {
+                const int i = V.tri[e] >> 8, j = V.tri[e] & 255;
+                G[i * ld + j] = (double)s_gamma(a, C[i * ld + j], i == j) + (i == j ? 1e-6 : 0.0);
+            }
+            ok = e_inverse_spd<W>(G, ld, reinterpret_cast<double*>(V.pw0), reinterpret_cast<double*>(V.pw1), V.tri, n,
+                                  t);
+            if (ok)  // in place: each element of G is read, then A written over it, by one thread
+                for (int e = t.tid; e < ntri; e += t.T) {
+                    const int i = V.tri[e] >> 8, j = V.tri[e] & 255;
+                    const float gi = (float)-G[i * ld + j];
+                    A[i * ld + j] = cscale(C[i * ld + j], gi);
                 }
+        } else {
+            for (int e = t.tid; e < ntri; e += t.T) {
+                const int i = V.tri[e] >> 8, j = V.tri[e] & 255;
+                const cfloat c = C[i * ld + j];
+                A[i * ld + j] = cscale(c, sqrtf(c.re * c.re + c.im * c.im));
+            }
         }
-        __syncwarp();
+        t.sync();
         if (ok) {
             // EMI: the eigenvalue nearest the shift 0.99; EVD: the largest in magnitude
-            cfloat* x = V.pw;
-            const float lambda = e_eigpair(A, n, ld, evd, V, x, lane);
-            {
+            cfloat* x = V.pw0;
+            const float lambda = e_eigpair<W>(A, n, ld, evd, V, x, t);
+            // the phasors of the pairs in place of C, by the warps that are free meanwhile
+            if (W == 1 || t.warp != 0) {
+                const int first = W == 1 ? 0 : 32;
+#pragma unroll 2
+                for (int e = t.tid - first; e < npairs; e += t.T - first) {
+                    cfloat& c = C[((V.tri[e] >> 8) + 1) * ld + (V.tri[e] & 255)];
+                    c = fphasor(c);
+                }
+            }
+            t.sync();
+            if (t.warp == 0) {
                 float s2 = 0.f;
                 for (int i = lane; i < n; i += 32) s2 += cabs2(x[i]);
                 s2 = warp_sum(s2);
@@ -387,15 +400,16 @@ __global__ void __launch_bounds__(32) k_eigh(PixArgs a, EighLayout L) {
                 // temporal coherence over pairs c < r, as the solvers compute it
                 float sre = 0.f, sim = 0.f;
                 int cnt = 0;
+#pragma unroll 4
                 for (int r = 1; r < n; ++r)
-                    for (int c = lane; c < r; c += 32) {
-                        const cfloat u = fphasor(C[r * ld + c]);
-                        const cfloat t = cconj(cmulc(cmul(u, w[c]), w[r]));
-                        if (!cisnan(t)) {
-                            sre += t.re;
-                            sim += t.im;
-                            ++cnt;
-                        }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int c = lane + 32 * h, cc = c < r ? c : 0;
+                        const cfloat v = cconj(cmulc(cmul(C[r * ld + cc], w[cc]), w[r]));
+                        const bool in = c < r && !cisnan(v);
+                        sre = in ? sre + v.re : sre;
+                        sim = in ? sim + v.im : sim;
+                        cnt += in;
                     }
                 sre = warp_sum(sre);
                 sim = warp_sum(sim);
@@ -408,8 +422,27 @@ __global__ void __launch_bounds__(32) k_eigh(PixArgs a, EighLayout L) {
                 }
             }
         }
-        if (lane == 0 && a.nc_flag) a.nc_flag[p] = 1;
-        __syncwarp();
+        if (t.tid == 0 && a.nc_flag) a.nc_flag[p] = 1;
+    }
+}
+
+// N > 16: four warps per pixel
+__global__ void __launch_bounds__(128, 8) k_eigh(PixArgs a, EighLayout L) {
+    extern __shared__ __align__(16) unsigned char eigh_smem[];
+    const EighCta<4> t{(int)threadIdx.x, (int)threadIdx.x & 31, (int)threadIdx.x >> 5};
+    eigh_pixels<4>(a, L, eigh_smem, blockIdx.x, gridDim.x, *a.nc_count, t);
+}
+
+// N <= 16: two warps per pixel while every pixel has a CTA of its own, else one warp per
+// pixel (the second one halves a pixel's latency but adds to its instructions)
+__global__ void __launch_bounds__(64, 12) k_eigh_small(PixArgs a, EighLayout L) {
+    extern __shared__ __align__(16) unsigned char eigh_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, count = *a.nc_count;
+    if (count <= (int)gridDim.x) {
+        eigh_pixels<2>(a, L, eigh_smem, blockIdx.x, gridDim.x, count, EighCta<2>{tid, lane, warp});
+    } else {
+        eigh_pixels<1>(a, L, eigh_smem + warp * L.bytes, 2 * blockIdx.x + warp, 2 * gridDim.x, count,
+                       EighCta<1>{lane, lane, 0});
     }
 }
 
@@ -690,19 +723,22 @@ static dpl_status launch_pixel64(const PixArgs& a, cudaStream_t s) {
     return check_launch("k_pixel64");
 }
 
-// Dense eigensolver over the listed non-converged pixels: one-warp CTAs, a persistent
-// grid of up to 8 per SM (the list length is known only on the device).
+// Dense eigensolver over the listed non-converged pixels, a grid of one resident wave (the
+// list length is known only on the device).
 static dpl_status launch_eigh(const PixArgs& a, cudaStream_t s) {
-    const EighLayout L = make_eigh_layout(a.n);
-    if (a.n > kEighMaxN || L.bytes > 227 * 1024)
+    const bool small = a.n <= kEighSmallN;
+    const EighLayout L = make_eigh_layout(a.n, small ? 2 : 4);
+    const size_t smem = small ? 2 * L.bytes : L.bytes;
+    if (a.n > kEighMaxN || smem > 227 * 1024)
         return fail(DPL_ERR_UNSUPPORTED, "eigensolver: N above 64 or shared memory above the SM limit");
+    const auto kernel = small ? k_eigh_small : k_eigh;
+    const int threads = small ? 64 : 128;
     int dev = 0, sms = 0, per_sm = 0;
     DPL_CUDA_TRY(cudaGetDevice(&dev));
     DPL_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    DPL_CUDA_TRY(cudaFuncSetAttribute(k_eigh, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes));
-    DPL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eigh, 32, L.bytes));
-    // one resident wave: each warp strides over the listed pixels
-    k_eigh<<<(unsigned)std::max(1, sms * std::max(1, per_sm)), 32, L.bytes, s>>>(a, L);
+    DPL_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DPL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    kernel<<<(unsigned)std::max(1, sms * std::max(1, per_sm)), threads, smem, s>>>(a, L);
     return check_launch("k_eigh");
 }
 
