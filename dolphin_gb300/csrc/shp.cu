@@ -7,12 +7,13 @@
 // at the edges), validity follows the unclamped origin and the window centre is always
 // False -- the reference's semantics.  The reference's float32 statistic
 // nslc * (2*log(pooled) - log(s1) - log(s2)) < threshold is, exactly,
-//     (s1 + s2)^2 < 4 exp(threshold / nslc) s1 s2,
-// which needs no logarithm: five float32 operations per (pixel, offset).  They carry
-// less than 5e-7 of relative error; where the two sides are within 2e-6 of each other,
-// the decision is taken in double precision on nslc * log1p((s1 - s2)^2 / (4 s1 s2))
-// (algebraically equal, no cancellation), so every mask bit is the exact comparison on
-// the float32 scale^2.  Scales whose products would overflow float32 and thresholds
+//     (s1 + s2)^2 < 4 c s1 s2,  c = exp(threshold / nslc),
+// which needs no logarithm: s2 has to lie within 2 sqrt(c (c - 1)) s1 of (2 c - 1) s1, two
+// subtractions per (pixel, offset).  They carry less than 2.7e-7 of the centre in error;
+// where the distance to the interval's end is within 5e-7 of it, the decision is taken in
+// double precision on nslc * log1p((s1 - s2)^2 / (4 s1 s2)) (algebraically equal, no
+// cancellation), so every mask bit is the exact comparison on the float32 scale^2.  Few
+// dates (c > 64) compare the two sides, within 2e-6 likewise.  Scales whose products would overflow float32 and thresholds
 // outside the usual range take the statistic with its logarithms (glrt_test), refined
 // in the same way where its rounding could reach the cutoff.
 //
@@ -30,10 +31,10 @@
 // with an equality (a tie decides by the walk's order) or with a non-finite sample is
 // walked step by step.  The decision is therefore bit-identical to the float64 walk.
 //
-// Both kernels gather a window row's decisions as bits, one item per (pixel, window
-// row, 32 offsets) with consecutive pixels on consecutive lanes (conflict-free reads of
-// the staged tile), and write the mask bytes of each output row afterwards, four per
-// store.
+// Both kernels gather the decisions as bits, consecutive pixels on consecutive lanes
+// (conflict-free reads of the staged tile): GLRT a pixel's whole window as one stream, KS
+// one item per (pixel, window row, 32 offsets).  The mask bytes of each output row are
+// written afterwards, up to 32 per store.
 #include <cuda.h>
 
 #include <algorithm>
@@ -121,12 +122,13 @@ __device__ __noinline__ bool glrt_test(float s1, float s2, float nslc, float thr
     return shp;
 }
 
-// Bytes (0/1) of an output row's masks from their bits: window row r (pixel by pixel) of
-// the tile row has its wx bits in the nw words at bits + r * nw, zero beyond wx; the
-// bytes go to dst[0 .. rows * wx).  C bytes (4, 8 or 16, at most wx + 1, so that they
-// touch two window rows at most) per aligned store.
+// Bytes (0/1) of an output row's masks from their bits: run r of the tile row (a pixel's
+// window row, or its whole window) has its wx bits in the nw words at bits + r * nw, zero
+// beyond wx; the bytes go to dst[0 .. rows * wx).  C bytes (4 to 32, at most wx + 1, so
+// that they touch two runs at most) per aligned store, by the threads t, t + nt, ...
 template <int C>
-__device__ __forceinline__ void write_masks(uint8_t* dst, const uint32_t* bits, int rows, int wx, int nw) {
+__device__ __forceinline__ void write_masks(uint8_t* dst, const uint32_t* bits, int rows, int wx, int nw, int t,
+                                            int nt) {
     const int len = rows * wx;
     const int head = min(len, (int)((C - (uint32_t)(reinterpret_cast<uintptr_t>(dst) & (C - 1))) & (C - 1)));
     const int chunks = (len - head) / C, tail = head + C * chunks;
@@ -135,7 +137,7 @@ __device__ __forceinline__ void write_masks(uint8_t* dst, const uint32_t* bits, 
         return (bits[r * nw + (wb >> 5)] >> (wb & 31)) & 1u;
     };
     const float inv_wx = 1.f / (float)wx;
-    for (int q = threadIdx.x; q < chunks; q += blockDim.x) {
+    for (int q = t; q < chunks; q += nt) {
         const int k = head + C * q;
         int r = (int)((float)k * inv_wx);  // k / wx: the float quotient is off by one at most
         int wb = k - r * wx;
@@ -149,30 +151,42 @@ __device__ __forceinline__ void write_masks(uint8_t* dst, const uint32_t* bits, 
         const uint32_t* w = bits + r * nw + (wb >> 5);
         const int sh = wb & 31, left = wx - wb;
         uint32_t v = w[0] >> sh;
-        if (sh > 32 - C && left > 32 - sh) v |= w[1] << (32 - sh);  // into the row's next word
-        if (left < C) v |= bits[(r + 1) * nw] << left;              // into the next window row
+        if (sh > 32 - C && left > 32 - sh) v |= w[1] << (32 - sh);  // into the run's next word
+        if (left < C) v |= bits[(r + 1) * nw] << left;              // into the next run
         uint32_t o[C / 4];
 #pragma unroll
         for (int i = 0; i < C / 4; ++i) o[i] = (((v >> (4 * i)) & 0xfu) * 0x00204081u) & 0x01010101u;
-        if constexpr (C == 16) *reinterpret_cast<uint4*>(dst + k) = make_uint4(o[0], o[1], o[2], o[3]);
+        if constexpr (C == 32)
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + k), "r"(o[0]), "r"(o[1]),
+                         "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7])
+                         : "memory");
+        else if constexpr (C == 16) *reinterpret_cast<uint4*>(dst + k) = make_uint4(o[0], o[1], o[2], o[3]);
         else if constexpr (C == 8) *reinterpret_cast<uint2*>(dst + k) = make_uint2(o[0], o[1]);
         else *reinterpret_cast<uint32_t*>(dst + k) = o[0];
     }
-    if ((int)threadIdx.x < head) dst[threadIdx.x] = (uint8_t)bit(threadIdx.x);
-    if ((int)threadIdx.x < len - tail) dst[tail + threadIdx.x] = (uint8_t)bit(tail + threadIdx.x);
+    if (t < head) dst[t] = (uint8_t)bit(t);  // head, len - tail < C <= nt
+    if (t < len - tail) dst[tail + t] = (uint8_t)bit(tail + t);
 }
 
-__device__ __forceinline__ void write_mask_row(uint8_t* dst, const uint32_t* bits, int rows, int wx, int nw) {
-    if (wx >= 15) write_masks<16>(dst, bits, rows, wx, nw);
-    else if (wx >= 7) write_masks<8>(dst, bits, rows, wx, nw);
-    else if (wx >= 3) write_masks<4>(dst, bits, rows, wx, nw);
+__device__ __forceinline__ void write_mask_row(uint8_t* dst, const uint32_t* bits, int rows, int wx, int nw, int t,
+                                               int nt) {
+    if (wx >= 31) write_masks<32>(dst, bits, rows, wx, nw, t, nt);
+    else if (wx >= 15) write_masks<16>(dst, bits, rows, wx, nw, t, nt);
+    else if (wx >= 7) write_masks<8>(dst, bits, rows, wx, nw, t, nt);
+    else if (wx >= 3) write_masks<4>(dst, bits, rows, wx, nw, t, nt);
     else
-        for (int k = threadIdx.x; k < rows; k += blockDim.x) dst[k] = (uint8_t)(bits[k] & 1u);  // wx == 1
+        for (int k = t; k < rows; k += nt) dst[k] = (uint8_t)(bits[k] & 1u);  // wx == 1
 }
 
-// Issue-bound.  1024 x 2048 pixels, 11 x 23 windows: 346 us (1.53 TB/s of mask bytes); a
-// logarithm per test and one byte per thread in the writes took 1098 us.
-__global__ void __launch_bounds__(256) k_glrt(const __grid_constant__ CUtensorMap tmap, GlrtArgs a) {
+// A pixel per thread, its window's bits one stream of words; 32 mask bytes per store.
+// Bound by instruction issue in the tests (~110 us) and by the mask bytes' stores (65 us),
+// which overlap in part: 1024 x 2048 pixels, 11 x 23 windows: 167 us (3.2 TB/s of mask
+// bytes).  The ratio test with an item per (pixel, window row) took 345 us, the interval
+// with such items and 16-byte stores 253, a logarithm per test and one byte per store
+// 1098.  kPlain (a window row is one word, every pixel has a thread of its own) drops the
+// loop over a row's words and the shared words' atomics: 212 -> 167 us.
+template <bool kPlain>
+__global__ void __launch_bounds__(256, 4) k_glrt(const __grid_constant__ CUtensorMap tmap, GlrtArgs a) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     // 128-byte aligned base (TMA destination), offset within the shared array so that
@@ -180,8 +194,8 @@ __global__ void __launch_bounds__(256) k_glrt(const __grid_constant__ CUtensorMa
     const uint32_t mis = (uint32_t)__cvta_generic_to_shared(smem_raw) & 127u;
     float* raw = reinterpret_cast<float*>(smem_raw + ((128u - mis) & 127u));
     const int n_tile = a.box_w * a.box_h;
-    uint32_t* bits = reinterpret_cast<uint32_t*>(raw + n_tile);  // [pixel][window row][nw]
-    const int wy = 2 * a.hy + 1, wx = 2 * a.hx + 1, nw = (wx + 31) >> 5;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(raw + n_tile);  // [pixel][nw]: its window's bits
+    const int wy = 2 * a.hy + 1, wx = 2 * a.hx + 1, W = wy * wx, nw = (W + 31) >> 5;
     const int or0 = blockIdx.y * a.tile_r, oc0 = blockIdx.x * a.tile_c;
     const int or1 = min(or0 + a.tile_r, a.out_rows), oc1 = min(oc0 + a.tile_c, a.out_cols);
     const int rr0 = clamp_start(a.sy / 2 + or0 * a.sy, a.hy, wy, a.rows);
@@ -225,62 +239,124 @@ __global__ void __launch_bounds__(256) k_glrt(const __grid_constant__ CUtensorMa
 
     const float nslc = (float)a.nslc;
     const int tc = oc1 - oc0, npix = (or1 - or0) * tc;
-    const int items = npix * wy * nw;
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-        const int rest = it / npix, pix = it - rest * npix;
-        const int word = rest / wy, wa = rest - word * wy;
+    // a pixel per thread; a small tile's pixels have their window rows spread over nsub
+    // threads, which share the words where one's rows end and the next one's begin
+    const int threads = blockDim.x, step = kPlain ? threads : min(npix, threads), nsub = kPlain ? 1 : threads / step;
+    const int sub = kPlain ? 0 : (int)threadIdx.x / step, pix0 = (int)threadIdx.x - sub * step;
+    const int wa0 = sub * wy / nsub, wa1 = sub < nsub ? (sub + 1) * wy / nsub : wa0;
+    if (nsub > 1) {
+        for (int i = threadIdx.x; i < npix * nw; i += threads) bits[i] = 0u;
+        __syncthreads();
+    }
+    for (int pix = pix0; wa0 < wa1 && pix < npix; pix += step) {
         const int pr = pix / tc;
         const int in_r = a.sy / 2 + (or0 + pr) * a.sy, in_c = a.sx / 2 + (oc0 + pix - pr * tc) * a.sx;
         const int r0 = clamp_start(in_r, a.hy, wy, a.rows), c0 = clamp_start(in_c, a.hx, wx, a.cols);
         const int ur0 = in_r - a.hy, uc0 = in_c - a.hx;
-        // valid window columns of the unclamped origin, within this word
-        const bool row_ok = (wa >= -ur0) && (wa < a.rows - ur0);
-        const int b0 = 32 * word, nb = min(wx - b0, 32);
-        const int v0 = max(max(0, -uc0) - b0, 0), v1 = row_ok ? min(min(wx, a.cols - uc0) - b0, nb) : 0;
-        uint32_t valid = v1 > v0 ? (v1 - v0 == 32 ? 0xffffffffu : ((1u << (v1 - v0)) - 1u) << v0) : 0u;
-        if (wa == a.hy && a.hx >= b0 && a.hx < b0 + 32) valid &= ~(1u << (a.hx - b0));
         const float s1 = raw[(in_r - rr0) * a.box_w + (in_c - x0)];
-        const float* row = raw + (r0 + wa - rr0) * a.box_w + (c0 - x0) + b0;
-        uint32_t shp = 0u, close = 0u;
-        if (!use_log) {
-            const float k1 = a.four_c * s1;
-            // each decision is the sign of a difference, shifted into a word (first offset
-            // highest); NaN differences are positive (canonical NaN)
-            auto test = [&](int wb) {
-                const float s2 = row[wb];
-                const float sum = s1 + s2;
-                const float r = k1 * s2;
-                const float diff = fmaf(sum, sum, -r);
-                // 1e-40 covers products that lose bits below the normal range
-                const float margin = fabsf(diff) - fmaf(2e-6f, r, 1e-40f);
-                shp = __funnelshift_l(__float_as_uint(diff), shp, 1);
-                close = __funnelshift_l(__float_as_uint(margin), close, 1);
-            };
-            int wb = 0;
-            for (; wb + 8 <= nb; wb += 8) {
+        const float* row = raw + (r0 + wa0 - rr0) * a.box_w + (c0 - x0);
+        const float center = a.center * s1, half = a.half * s1, margin = fmaf(5e-7f, center, 1e-40f);
+        const float k1 = a.four_c * s1;
+        // valid window columns v0 .. v1 - 1 and rows of the unclamped origin
+        const int v0 = max(0, -uc0), v1 = min(wx, a.cols - uc0);
+        const auto columns = [&](int b0, int nb) {
+            const int lo = max(v0 - b0, 0), hi = min(v1 - b0, nb);
+            return hi > lo ? (0xffffffffu >> (32 - (hi - lo))) << lo : 0u;
+        };
+        const uint32_t first = columns(0, min(wx, 32));
+        // the bits of the rows so far, from word `w` of the pixel on
+        uint32_t* w = bits + pix * nw + (wa0 * wx >> 5);
+        uint64_t acc = 0u;
+        int fill = wa0 * wx & 31;
+        const auto flush = [&](uint32_t v) {
+            if (nsub > 1) atomicOr(w, v);
+            else *w = v;
+            ++w;
+        };
+        for (int wa = wa0; wa < wa1; ++wa, row += a.box_w) {
+            const bool row_ok = (wa >= -ur0) && (wa < a.rows - ur0);
+            const float* span = row;
+            for (int b0 = 0; b0 < (kPlain ? 1 : wx); b0 += 32, span += 32) {
+                const int nb = kPlain ? wx : min(wx - b0, 32);
+                uint32_t valid = row_ok ? (b0 ? columns(b0, nb) : first) : 0u;
+                if (wa == a.hy && a.hx >= b0 && a.hx < b0 + 32) valid &= ~(1u << (a.hx - b0));
+                uint32_t shp = 0u;
+                if (!use_log && a.interval) {
+                    // each decision is the sign of a difference, shifted into a word (first offset
+                    // highest); NaN differences are positive (canonical NaN)
+                    float nearest = INFINITY;
+                    auto distance = [&](int wb) { return fabsf(span[wb] - center) - half; };
+                    auto test = [&](int wb) {
+                        const float d = distance(wb);
+                        shp = __funnelshift_l(__float_as_uint(d), shp, 1);
+                        nearest = fminf(nearest, fabsf(d));
+                    };
+                    int wb = 0;
+                    for (; wb + 8 <= nb; wb += 8) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) test(wb + i);
-            }
+                        for (int i = 0; i < 8; ++i) test(wb + i);
+                    }
+                    if (nb & 4) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) test(wb + i);
+                        wb += 4;
+                    }
+                    if (nb & 2) {
+                        test(wb);
+                        test(wb + 1);
+                        wb += 2;
+                    }
+                    if (nb & 1) test(wb);
+                    shp = __brev(shp) >> (32 - nb);
+                    if (nearest <= margin) {
 #pragma unroll 1
-            for (; wb < nb; ++wb) test(wb);
-            shp = __brev(shp) >> (32 - nb);
-            close = __brev(close) >> (32 - nb);
-            close &= valid;
-            while (close) {
-                const int wb2 = __ffs(close) - 1;
-                close &= close - 1u;
-                shp = (shp & ~(1u << wb2)) | (uint32_t)glrt_exact(s1, row[wb2], nslc, a.thr) << wb2;
+                        for (int i = 0; i < nb; ++i)
+                            if ((valid >> i & 1u) && fabsf(distance(i)) <= margin)
+                                shp = (shp & ~(1u << i)) | (uint32_t)glrt_exact(s1, span[i], nslc, a.thr) << i;
+                    }
+                } else if (!use_log) {
+                    uint32_t close = 0u;
+#pragma unroll 4
+                    for (int wb = 0; wb < nb; ++wb) {
+                        const float s2 = span[wb];
+                        const float sum = s1 + s2;
+                        const float r = k1 * s2;
+                        const float diff = fmaf(sum, sum, -r);
+                        // 1e-40 covers products that lose bits below the normal range
+                        const float gap = fabsf(diff) - fmaf(2e-6f, r, 1e-40f);
+                        shp = __funnelshift_l(__float_as_uint(diff), shp, 1);
+                        close = __funnelshift_l(__float_as_uint(gap), close, 1);
+                    }
+                    shp = __brev(shp) >> (32 - nb);
+                    close = __brev(close) >> (32 - nb);
+                    close &= valid;
+                    while (close) {
+                        const int wb2 = __ffs(close) - 1;
+                        close &= close - 1u;
+                        shp = (shp & ~(1u << wb2)) | (uint32_t)glrt_exact(s1, span[wb2], nslc, a.thr) << wb2;
+                    }
+                } else {
+                    for (int wb = 0; wb < nb; ++wb)
+                        if ((valid >> wb) & 1u) shp |= (uint32_t)glrt_test(s1, span[wb], nslc, a.thr) << wb;
+                }
+                acc |= (uint64_t)(shp & valid) << fill;
+                fill += nb;
+                if (fill >= 32) {
+                    flush((uint32_t)acc);
+                    acc >>= 32;
+                    fill -= 32;
+                }
             }
-        } else {
-            for (int wb = 0; wb < nb; ++wb)
-                if ((valid >> wb) & 1u) shp |= (uint32_t)glrt_test(s1, row[wb], nslc, a.thr) << wb;
         }
-        bits[(pix * wy + wa) * nw + word] = shp & valid;
+        if (fill > 0) flush((uint32_t)acc);
     }
     __syncthreads();
-    for (int orow = or0; orow < or1; ++orow)
-        write_mask_row(a.is_shp + ((int64_t)orow * a.out_cols + oc0) * (wy * wx), bits + (orow - or0) * tc * wy * nw,
-                       tc * wy, wx, nw);
+    // an output row per warp, or (few rows) the CTA on one after the other
+    const bool by_warp = 32 * (or1 - or0) >= threads;
+    const int first_row = by_warp ? (int)threadIdx.x >> 5 : 0, row_step = by_warp ? threads >> 5 : 1;
+    for (int r = first_row; r < or1 - or0; r += row_step)
+        write_mask_row(a.is_shp + ((int64_t)(or0 + r) * a.out_cols + oc0) * W, bits + r * tc * nw, tc, W, nw,
+                       by_warp ? threadIdx.x & 31 : threadIdx.x, by_warp ? 32 : threads);
 }
 
 // ---------------------------------------------------------------------------------
@@ -413,7 +489,7 @@ __global__ void __launch_bounds__(256) k_ks(const __grid_constant__ KsArgs a) {
     __syncthreads();
     for (int orow = or0; orow < or1; ++orow)
         write_mask_row(a.is_shp + ((int64_t)orow * a.out_cols + oc0) * (wy * wx), bits + (orow - or0) * tc * wy * nw,
-                       tc * wy, wx, nw);
+                       tc * wy, wx, nw, threadIdx.x, blockDim.x);
 }
 
 template <int NS>
@@ -482,6 +558,13 @@ dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_
     const double c = nslc > 0 ? std::exp((double)threshold / nslc) : 0.0;
     a.ratio = threshold > 0.f && c > 1.0 && c < 1e12;
     a.four_c = a.ratio ? (float)(4.0 * c) : 0.f;
+    // the interval of s2 / s1: 2 c - 1 -+ 2 sqrt(c (c - 1)).  Its lower end is 1 / (4 c), and
+    // the error bound of its test a part of the centre: up to c = 64 the two stay two orders
+    // of magnitude apart (beyond, as with one or two dates, the ratio test)
+    const double cm1 = nslc > 0 ? std::expm1((double)threshold / nslc) : 0.0;
+    a.interval = a.ratio && c <= 64.0;
+    a.center = a.interval ? (float)(2.0 * c - 1.0) : 0.f;
+    a.half = a.interval ? (float)(2.0 * std::sqrt(c * cm1)) : 0.f;
     a.ratio_max = a.ratio ? (float)std::sqrt(1e37 / (4.0 * c)) : 0.f;
     if (a.out_rows == 0 || a.out_cols == 0) return DPL_OK;
     // pick the largest tile whose TMA box fits the 256-element box limit and ~96 KB smem
@@ -493,7 +576,7 @@ dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_
     // staged scale^2, then the tile's mask bits
     auto smem_for = [&](int r, int c) {
         return (size_t)box_w(c) * box_h(r) * sizeof(float) + 128 +
-               (size_t)r * c * wy * ((wx + 31) / 32) * sizeof(uint32_t);
+               (size_t)r * c * ((wy * wx + 31) / 32) * sizeof(uint32_t);
     };
     while (smem_for(tr, tc) > 96 * 1024 && (tr > 1 || tc > 1)) {
         if (tr >= tc && tr > 1) tr /= 2;
@@ -519,8 +602,11 @@ dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_
     const size_t smem = smem_for(tr, tc);
     if (smem > (size_t)227 * 1024) return fail(DPL_ERR_UNSUPPORTED, "GLRT window too large for shared memory");
     dim3 grid(ceil_div(a.out_cols, tc), ceil_div(a.out_rows, tr));
-    DPL_CUDA_TRY(cudaFuncSetAttribute(k_glrt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_glrt<<<grid, 256, smem, s>>>(map, a);
+    // one word per window row and a pixel per thread
+    const bool plain = wx <= 32 && std::min(tr, a.out_rows) * std::min(tc, a.out_cols) >= 256;
+    const auto kernel = plain ? k_glrt<true> : k_glrt<false>;
+    DPL_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, 256, smem, s>>>(map, a);
     return check_launch("k_glrt");
 }
 

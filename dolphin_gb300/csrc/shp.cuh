@@ -15,9 +15,11 @@ struct GlrtArgs {
     int tile_r, tile_c;  // output pixels per CTA
     int box_w, box_h;    // TMA box (floats x rows)
     uint8_t* is_shp;     // (out_rows, out_cols, wy, wx) bytes
-    int ratio;           // the ratio test applies (else logarithms)
+    int ratio;           // no logarithms: the ratio test applies,
+    int interval;        //   as an interval of s2
     float four_c;        // 4 exp(thr / nslc)
-    float ratio_max;     // largest scale^2 of the ratio test
+    float center, half;  // the interval of s2 / s1
+    float ratio_max;     // largest scale^2 of either test
     int* status;         // set to DPL_ERR_TIMEOUT if a bounded wait gives up
 };
 

@@ -119,3 +119,23 @@ def test_glrt_threshold_is_the_quantile():
 
     for alpha in [0.0, 1e-12, 1e-5, 0.001, 0.01, 0.05, 0.3, 0.9, 1.0]:
         assert glrt_threshold(alpha) == float(stats.chi2.ppf(1 - alpha, df=1))
+
+
+@gpu
+@pytest.mark.parametrize("nslc", [3, 4, 30, 1000])
+@pytest.mark.parametrize("hx", [0, 1, 3, 7, 11, 14, 15, 16, 31])
+def test_glrt_interval_ends(nslc, hx):
+    """Scales within a few float32 steps of the interval's two ends, at every remainder of a
+    window row's offsets: each decision is the float64 one."""
+    dp = _dp()
+    rng = np.random.default_rng(nslc + hx)
+    rows, cols = 19, 70
+    c = np.exp(10.827566170662733 / nslc)  # the 0.999 quantile of chi2(1)
+    end = 2 * c - 1 + 2 * np.sqrt(c * (c - 1))
+    level = end ** rng.integers(0, 3, size=(rows, cols))
+    var = (2 * level * (1 + rng.integers(-6, 7, size=level.shape) * 2.0**-24)).astype(np.float32)
+    mean = np.zeros_like(var)
+    got = dp.estimate_neighbors(halfwin_rowcol=(2, hx), mean=mean, var=var, nslc=nslc, alpha=0.001)
+    want = O.estimate_neighbors_glrt(mean, var, (2, hx), (1, 1), nslc, 0.001, exact=True)
+    np.testing.assert_array_equal(got, want)
+    assert want.any()
