@@ -32,9 +32,9 @@
 // walked step by step.  The decision is therefore bit-identical to the float64 walk.
 //
 // Both kernels gather the decisions as bits, consecutive pixels on consecutive lanes
-// (conflict-free reads of the staged tile): GLRT a pixel's whole window as one stream, KS
-// one item per (pixel, window row, 32 offsets).  The mask bytes of each output row are
-// written afterwards, up to 32 per store.
+// (conflict-free reads of the staged tile): a pixel's whole window is one stream, filled
+// by the pixel's thread (GLRT) or by items of 32 offsets of a window row (KS).  The mask
+// bytes of each output row are written afterwards, up to 32 per store.
 #include <cuda.h>
 
 #include <algorithm>
@@ -424,8 +424,8 @@ __device__ __noinline__ bool ks_walk(const float* x1, const float* x2, int n, co
 template <int NS>
 __global__ void __launch_bounds__(256) k_ks(const __grid_constant__ KsArgs a) {
     extern __shared__ float samp[];  // sorted samples [pixel][np], then the mask bits
-    const int n = a.n, np = a.n | 1, d = a.n - a.ns;
-    const int wy = 2 * a.hy + 1, wx = 2 * a.hx + 1, nw = (wx + 31) >> 5;
+    const int n = a.n, np = a.pitch, d = a.n - a.ns;
+    const int wy = 2 * a.hy + 1, wx = 2 * a.hx + 1, W = wy * wx, nw = (wx + 31) >> 5, pw = (W + 31) >> 5;
     const int or0 = blockIdx.y * a.tile_r, oc0 = blockIdx.x * a.tile_c;
     const int or1 = min(or0 + a.tile_r, a.out_rows), oc1 = min(oc0 + a.tile_c, a.out_cols);
     // input region of the (unclamped) windows, intersected with the image
@@ -443,9 +443,10 @@ __global__ void __launch_bounds__(256) k_ks(const __grid_constant__ KsArgs a) {
             asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + c * np)), "l"(src + c)
                          : "memory");
     }
+    const int tc = oc1 - oc0, npix = (or1 - or0) * tc;
+    for (int i = threadIdx.x; i < npix * pw; i += blockDim.x) bits[i] = 0u;
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const int tc = oc1 - oc0, npix = (or1 - or0) * tc;
     const int items = npix * wy * nw;
     for (int it = threadIdx.x; it < items; it += blockDim.x) {
         const int rest = it / npix, pix = it - rest * npix;
@@ -484,12 +485,17 @@ __global__ void __launch_bounds__(256) k_ks(const __grid_constant__ KsArgs a) {
             }
             if (wa == a.hy && a.hx >= b0 && a.hx < b0 + 32) shp &= ~(1u << (a.hx - b0));
         }
-        bits[(pix * wy + wa) * nw + word] = shp;
+        if (shp) {  // into the pixel's stream, whose words the rows share
+            const int at = wa * wx + 32 * word, sh = at & 31;
+            uint32_t* w = bits + pix * pw + (at >> 5);
+            atomicOr(w, shp << sh);
+            if (sh && shp >> (32 - sh)) atomicOr(w + 1, shp >> (32 - sh));
+        }
     }
     __syncthreads();
     for (int orow = or0; orow < or1; ++orow)
-        write_mask_row(a.is_shp + ((int64_t)orow * a.out_cols + oc0) * (wy * wx), bits + (orow - or0) * tc * wy * nw,
-                       tc * wy, wx, nw, threadIdx.x, blockDim.x);
+        write_mask_row(a.is_shp + ((int64_t)orow * a.out_cols + oc0) * W, bits + (orow - or0) * tc * pw, tc, W, pw,
+                       threadIdx.x, blockDim.x);
 }
 
 template <int NS>
@@ -583,6 +589,9 @@ dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_
         else tc /= 2;
     }
     if (box_w(tc) > 256 || box_h(tr) > 256) return fail(DPL_ERR_UNSUPPORTED, "GLRT window too large for a TMA box");
+    // the interface's limit, well above one pixel's needs here
+    if ((size_t)2 * box_w(1) * box_h(1) * sizeof(float) + 128 + (size_t)wy * wx > 227 * 1024)
+        return fail(DPL_ERR_UNSUPPORTED, "GLRT window too large for shared memory");
     a.tile_r = tr;
     a.tile_c = tc;
     a.box_w = box_w(tc);
@@ -600,7 +609,6 @@ dpl_status launch_glrt(const float* mean, const float* var, int64_t rows, int64_
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(DPL_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
     const size_t smem = smem_for(tr, tc);
-    if (smem > (size_t)227 * 1024) return fail(DPL_ERR_UNSUPPORTED, "GLRT window too large for shared memory");
     dim3 grid(ceil_div(a.out_cols, tc), ceil_div(a.out_rows, tr));
     // one word per window row and a pixel per thread
     const bool plain = wx <= 32 && std::min(tr, a.out_rows) * std::min(tc, a.out_cols) >= 256;
@@ -746,17 +754,21 @@ extern "C" dpl_status dpl_shp_ks(const float* amp_stack, int64_t nslc, int64_t r
     // two CTAs per SM; windows too large for that get what one CTA can hold
     int tr = 8, tc = 32;
     auto region = [&](int r, int c) { return ((size_t)(r - 1) * sy + wy) * ((size_t)(c - 1) * sx + wx); };
-    auto smem_for = [&](int r, int c) {
-        return region(r, c) * (n | 1) * sizeof(float) + (size_t)r * c * wy * ((wx + 31) / 32) * sizeof(uint32_t);
+    const auto bytes_for = [&](int r, int c, int pitch) {
+        return region(r, c) * pitch * sizeof(float) + (size_t)r * c * ((wy * wx + 31) / 32) * sizeof(uint32_t);
     };
+    if (2 * (n + 1) * sizeof(int) + region(1, 1) * n * sizeof(float) > 200 * 1024)
+        return fail(DPL_ERR_UNSUPPORTED, "dpl_shp_ks: window too large");
+    // an odd pitch (no bank conflicts) wherever one pixel's window has room for it
+    a.pitch = bytes_for(1, 1, n | 1) <= 227 * 1024 ? n | 1 : n;
+    const auto smem_for = [&](int r, int c) { return bytes_for(r, c, a.pitch); };
     while (smem_for(tr, tc) > 110 * 1024 && (tr > 1 || tc > 1)) {
         if (tr * sy >= tc * sx && tr > 1) tr /= 2;
         else if (tc > 1) tc /= 2;
         else tr /= 2;
     }
-    if (smem_for(tr, tc) > 227 * 1024) return fail(DPL_ERR_UNSUPPORTED, "dpl_shp_ks: window too large");
     a.tile_r = tr;
     a.tile_c = tc;
-    a.off_bits = (int)region(tr, tc) * (n | 1);
+    a.off_bits = (int)region(tr, tc) * a.pitch;
     return launch_ks<4>(a, dim3(ceil_div(out_cols, tc), ceil_div(out_rows, tr)), smem_for(tr, tc), s);
 }

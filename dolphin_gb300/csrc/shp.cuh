@@ -28,6 +28,7 @@ struct KsArgs {
     int8_t lo[kMaxNslc + 1], hi[kMaxNslc + 1];  // admissible i2 per i1 of the merge walk
     int8_t env_lo[kMaxNslc], env_hi[kMaxNslc];  // envelope of sample t: indices into x1 (-1: none)
     int ns;               // samples with a lower bound (n minus the first index that has one)
+    int pitch;            // floats per pixel's samples in shared memory
     int off_bits;         // the mask bits, in 4-byte words from the start of shared memory
     int n, rows, cols, hy, hx, sy, sx, out_rows, out_cols;
     int tile_r, tile_c;

@@ -139,3 +139,23 @@ def test_glrt_interval_ends(nslc, hx):
     want = O.estimate_neighbors_glrt(mean, var, (2, hx), (1, 1), nslc, 0.001, exact=True)
     np.testing.assert_array_equal(got, want)
     assert want.any()
+
+
+@gpu
+@pytest.mark.parametrize("n,hw", [(2, (78, 79)), (4, (55, 56)), (1, (400, 1))])
+def test_ks_windows_at_the_limit(n, hw):
+    """Windows whose samples fill shared memory: the unpadded pitch, one pixel per CTA."""
+    dp = _dp()
+    rng = np.random.default_rng(n)
+    # every third pixel, the first one with a whole window
+    r, c = (1 + 3 * ((h + 1) // 3) for h in hw)
+    rows, cols = r + hw[0] + 4, c + hw[1] + 5
+    amp = rng.rayleigh(3.0, size=(n, rows, cols)).astype(np.float32)
+    got = dp.estimate_neighbors(halfwin_rowcol=hw, strides=dp.Strides(3, 3), amp_stack=amp, alpha=0.05, method="ks")
+    x = np.sort(amp, axis=0)
+    win = x[:, r - hw[0]:r + hw[0] + 1, c - hw[1]:c + hw[1] + 1]
+    want = O.ks_max_cdf_dist(np.broadcast_to(x[:, r, c], (win[0].size, n)), win.reshape(n, -1).T) < \
+        O.ks_critical_distance(n, 0.05)
+    want = want.reshape(win.shape[1:])
+    want[hw] = False
+    np.testing.assert_array_equal(got[r // 3, c // 3], want)
