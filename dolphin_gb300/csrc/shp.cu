@@ -419,7 +419,7 @@ __device__ __noinline__ bool ks_walk(const float* x1, const float* x2, int n, co
 // s < ns = n - d, NS being ns rounded up to a multiple of 4.  The samples of a pixel are
 // contiguous in shared memory (immediate offsets), at an odd pitch (consecutive pixels
 // fall into different banks).  Issue-bound (63 % of issue slots): 512 x 512 pixels, 20
-// dates, 11 x 23 windows, 300 us; a merge walk per thread, divergent and with bank
+// dates, 11 x 23 windows, 313 us; a merge walk per thread, divergent and with bank
 // conflicts, took 3949 us.
 template <int NS>
 __global__ void __launch_bounds__(256) k_ks(const __grid_constant__ KsArgs a) {

@@ -29,7 +29,7 @@
 // order: phases, CRLB and estimator are the same bit for bit.  One pixel-warp at K = 30,
 // alone on the SM: a real sweep 2594 -> 2041 cycles, the Hermitian one 6982 -> 5268.
 //
-// 1034 x 1046 pixels at N = 30: 17.3 -> 14.2 ms.
+// 1034 x 1046 pixels at N = 30: 17.3 -> 13.9 ms.
 //
 // Register rotation keeps the sweeps in compact loops: before the steps k, k + 1 (k
 // even), slot s of a row holds column (k + s) mod K, so the pivot columns are slots 0 and
