@@ -163,6 +163,28 @@ __device__ __forceinline__ float sim_phase(const SimPrepArgs& a, int t, int64_t 
     return a.stack[(int64_t)t * a.npix + p];
 }
 
+// exp(i angle z), and z's components added to the sums of nan_to_num(z).  In the ordinary
+// range z / |z|, the reciprocal root refined by one Newton step (components to 2e-7 of
+// their own size); zeros, NaN, infinities and extreme magnitudes by way of the angle.
+// (By way of the angle throughout, the two functions' instructions bounded k_sim_prep:
+// 30 layers of 1400 x 1500 pixels 230 us, 142 us now, 7.1 TB/s.)
+__device__ __forceinline__ float2 sim_phasor(float2 z, float& sre, float& sim) {
+    const float s = fmaf(z.x, z.x, z.y * z.y);
+    float2 u;
+    if (s > 1e-30f && s < 1e30f) {
+        float r = rsqrtf(s);
+        r = fmaf(0.5f * r, fmaf(-s * r, r, 1.f), r);
+        u = make_float2(z.x * r, z.y * r);
+        sre = fadd(sre, z.x);
+        sim = fadd(sim, z.y);
+    } else {
+        sincosf(atan2f(z.y, z.x), &u.y, &u.x);
+        sre = fadd(sre, nan_to_num_f(z.x));
+        sim = fadd(sim, nan_to_num_f(z.y));
+    }
+    return u;
+}
+
 __global__ void __launch_bounds__(256) k_sim_prep(SimPrepArgs a) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.npix) return;
@@ -171,20 +193,28 @@ __global__ void __launch_bounds__(256) k_sim_prep(SimPrepArgs a) {
     float sre = 0.f, sim = 0.f;
     if (!a.nearest) {
         // one pass: sums and phasors; a pixel found invalid is overwritten with NaN
-        for (int t = 0; t < a.nin; ++t) {
-            float ph;
-            if (a.is_complex) {
-                const float2 z = reinterpret_cast<const float2*>(a.stack)[(int64_t)t * a.npix + p];
-                sre = fadd(sre, nan_to_num_f(z.x));
-                sim = fadd(sim, nan_to_num_f(z.y));
-                ph = atan2f(z.y, z.x);
-            } else {
-                ph = a.stack[(int64_t)t * a.npix + p];
-                sre = fadd(sre, nan_to_num_f(ph));
+        if (a.is_complex) {
+            const float2* __restrict__ z = reinterpret_cast<const float2*>(a.stack) + p;
+            float2* __restrict__ out = a.unit + p;
+            for (int t0 = 0; t0 < a.nin; t0 += 4) {
+                float2 v[4];  // four layers' loads in flight
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = z[(int64_t)min(t0 + i, a.nin - 1) * a.npix];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (t0 + i >= a.nin) break;
+                    const float2 u = sim_phasor(v[i], sre, sim);
+                    out[(int64_t)(t0 + i) * a.npix] = masked ? make_float2(qnan, qnan) : u;
+                }
             }
-            float2 u = make_float2(qnan, qnan);
-            if (!masked) sincosf(ph, &u.y, &u.x);
-            a.unit[(int64_t)t * a.npix + p] = u;
+        } else {
+            for (int t = 0; t < a.nin; ++t) {
+                const float ph = a.stack[(int64_t)t * a.npix + p];
+                sre = fadd(sre, nan_to_num_f(ph));
+                float2 u = make_float2(qnan, qnan);
+                if (!masked) sincosf(ph, &u.y, &u.x);
+                a.unit[(int64_t)t * a.npix + p] = u;
+            }
         }
         const bool ok = !(sre == 0.f && sim == 0.f) && !masked;
         a.valid[p] = ok ? 1 : 0;
