@@ -531,8 +531,8 @@ def run_ours(args, rank, world, pool, cores):
         cpu = {"value": cv, "unit": UNIT, "cores": cores, "kind": "port",
                "sample": cd + " (numpy restatement of the reference algorithm)"}
     # per block: k_ps_block, k_glrt_scale, k_glrt, k_prep, k_cov_tc, k_solve_reg, k_pixel (LU list),
-    # k_eigh (pixels that missed the stopping rule), k_post
-    launches_per_step = len(plan) * 9
+    # k_eigh (pixels that missed the stopping rule), k_pixel (those it cannot take), k_post
+    launches_per_step = len(plan) * 10
     b_pl = 8 * NSLC + 8 + 2 + 8 * NSLC + 4 + 2 + 4 + 1 + 4 * NSLC + 4 * (NSLC - 2)
     hbm_peak = float(peaks.get("hbm_gbs", 6768.8))
     e2e_rate = px / (e2e_ms / 1000.0)

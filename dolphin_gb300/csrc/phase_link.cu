@@ -312,7 +312,8 @@ __device__ __forceinline__ void eigh_pixels(const PixArgs& a, const EighLayout& 
     for (int i = t.tid; i < n; i += t.T)
         for (int j = 0; j <= i; ++j) V.tri[i * (i + 1) / 2 + j] = (unsigned short)(i << 8 | j);
     for (; idx < count; idx += stride) {
-        const int64_t p = a.nc_list[idx];
+        const int entry = a.nc_list[idx];
+        const int64_t p = entry < 0 ? ~entry : entry;
         t.sync();
         // the coherence, normalised as the solvers read it
         if (a.Cplanar) {
@@ -422,7 +423,11 @@ __device__ __forceinline__ void eigh_pixels(const PixArgs& a, const EighLayout& 
                 }
             }
         }
-        if (t.tid == 0 && a.nc_flag) a.nc_flag[p] = 1;
+        if (t.tid == 0) {
+            if (a.nc_flag) a.nc_flag[p] = 1;
+            // |Gamma| not positive definite: the solver's last iterate stays, where it has one
+            if (!ok && entry < 0) a.redo_list[atomicAdd(a.redo_count, 1)] = (int)p;
+        }
     }
 }
 
@@ -742,15 +747,16 @@ static dpl_status launch_eigh(const PixArgs& a, cudaStream_t s) {
     return check_launch("k_eigh");
 }
 
-// Solve pass, then the LU pass over the pixels it lists (`fb`: a counter, then room
+// Solve pass, then the LU pass over the pixels it lists (`fb`: two counters, then room
 // for every pixel index) and, with `nc` (the same shape), the dense eigensolver over
-// the pixels whose iteration missed its stopping rule.
+// the pixels whose iteration missed its stopping rule; last, the LU pass's iterates of the
+// few that neither of them solved (listed where the first list was).
 template <int MODE>
 static dpl_status launch_pixel(PixArgs& a, cudaStream_t s, int* fb = nullptr, int* nc = nullptr) {
     if (a.npix == 0) return DPL_OK;
     if (MODE == kCovOnly) return launch_pixel_pass<MODE, false>(a, s);
     if (!fb) return fail(DPL_ERR_WORKSPACE, "solver: missing fallback list");
-    DPL_CUDA_TRY(cudaMemsetAsync(fb, 0, sizeof(int), s));
+    DPL_CUDA_TRY(cudaMemsetAsync(fb, 0, 2 * sizeof(int), s));
     a.fb_count = fb;
     a.fb_list = fb + 64;
     // non-converged pixels are listed (and solved again) only where the coherence is stored
@@ -766,7 +772,14 @@ static dpl_status launch_pixel(PixArgs& a, cudaStream_t s, int* fb = nullptr, in
     b.list_count = a.fb_count;
     st = launch_pixel_pass<MODE, true>(b, s);
     if (st != DPL_OK || !a.nc_count) return st;
-    return launch_eigh(a, s);
+    a.redo_count = fb + 1;
+    a.redo_list = fb + 64;
+    st = launch_eigh(a, s);
+    if (st != DPL_OK) return st;
+    b.list = a.redo_list;
+    b.list_count = a.redo_count;
+    b.nc_list = nullptr;  // every step, nothing listed
+    return launch_pixel_pass<MODE, true>(b, s);
 }
 
 // Tensor-core covariance: fills `Cg` (npix x n*n planar floats).

@@ -82,8 +82,11 @@ struct PixArgs {
     int* ill_list;           // register solver: ill-conditioned pixels for the plain form (null: not listed)
     int* ill_count;
     int lanes;               // register solver: threads per pixel (8, 16, 32; 0 = the smallest that fits)
-    int* nc_list;            // pixels whose eigen-iteration missed its stopping rule (null: not listed)
+    int* nc_list;            // pixels whose eigen-iteration missed its stopping rule (null: not listed);
+                             // ~pixel where the LU pass left the iterate out
     int* nc_count;
+    int* redo_list;          // of those, the pixels that the dense eigensolver cannot take (LU pass again)
+    int* redo_count;
     uint8_t* nc_flag;        // (npix) 1 where the dense eigensolver replaced the iterate, or null
     int eigh;                // FP64 form: the dense eigensolver for iterations that miss the rule
     int slots;               // register solver: row slots K (even, >= n; 0 = n rounded up to even)

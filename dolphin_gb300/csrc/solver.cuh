@@ -429,7 +429,7 @@ __device__ void solve_pixel(const PixArgs& a, int64_t p, const SolveMats& m, int
 #pragma unroll
     for (int q = 0; q < NB; ++q) v[q] = lane + 32 * q < n ? cmake(inv_sqrt_n, 0.f) : cmake(0.f, 0.f);
     float lambda;
-    bool converged;
+    bool converged, stalled = false;
     if (!evd) {
         if (!kLU) {
             // packed A - 0.99 I, complex Cholesky, inverse iteration
@@ -483,10 +483,10 @@ __device__ void solve_pixel(const PixArgs& a, int64_t p, const SolveMats& m, int
             // a pixel that the dense eigensolver takes over needs no iterate: most listed
             // pixels use all 49 steps, 1.4 M of the pass's 1.65 M cycles at N = 30 (the pass
             // on 1034 x 1046 pixels: 806 -> 353 us; at N = 10 on 128 x 128: 156 -> 60 us)
-            if (a.nc_list && s_lu_stalls<NB>(A, n, src, A + n * n, m.v, lane))
-                converged = false;
-            else
-                converged = s_iterate<NB>(v, [&](cfloat(&x)[NB]) { s_lu_solve<NB>(A, n, src, x, lane); });
+            // (it takes over all but those whose |Gamma| is not positive definite in double:
+            // these come back in a pass of their own, which iterates)
+            stalled = a.nc_list && s_lu_stalls<NB>(A, n, src, A + n * n, m.v, lane);
+            converged = !stalled && s_iterate<NB>(v, [&](cfloat(&x)[NB]) { s_lu_solve<NB>(A, n, src, x, lane); });
             s_publish<NB>(m.v, v, n, lane);
             float s = 0.f;
 #pragma unroll
@@ -557,7 +557,7 @@ __device__ void solve_pixel(const PixArgs& a, int64_t p, const SolveMats& m, int
         a.eig[p] = lambda;
         a.est[p] = evd ? 0 : 1;
         // the stopping rule not met within 49 steps: listed for the dense eigensolver
-        if (!converged && a.nc_list) a.nc_list[atomicAdd(a.nc_count, 1)] = (int)p;
+        if (!converged && a.nc_list) a.nc_list[atomicAdd(a.nc_count, 1)] = stalled ? ~(int)p : (int)p;
     }
     // temporal coherence over pairs i < j: phasor(C_ij) conj(phasor(v_i conj v_j)),
     // with C_ij = conj(C_ji) (packed (j, i)) and phasor(v_i conj v_j) = w_i conj(w_j)
