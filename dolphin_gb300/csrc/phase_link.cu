@@ -893,6 +893,10 @@ static dpl_status launch_cov_tc_batch(std::vector<TcArgs> items, bool tf32, int*
     }
     TcArgs carve{};
     tc_carve(carve, nst, nmax, kpad, kwords, npass, tf32);
+    if (carve.smem_bytes > 227 * 1024) {  // as in tc_configure: without the odd number of words
+        for (TcArgs& t : items) t.kwords = t.kpad / 32;
+        tc_carve(carve, nst, nmax, kpad, kpad / 32, npass, tf32);
+    }
     if (carve.smem_bytes > 227 * 1024) return fail(DPL_ERR_UNSUPPORTED, "batch: covariance shared memory exceeds the SM limit");
     TcBatch b{};
     b.nitems = (int)items.size();
