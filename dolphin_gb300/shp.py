@@ -31,8 +31,26 @@ def ks_critical_distance(nslc: int, alpha: float) -> float:
     Scans distances from 0.01 in steps of 0.001 and returns the first whose
     Kolmogorov-series p-value (100 terms, N/2 effective samples) is <= alpha.
     """
-    0.11 / math.sqrt(nslc / 2.0)  # raises for nslc <= 0, as the reference does
-    return float(_lib.load().dpl_ks_critical_distance(int(nslc), float(alpha)))
+    sq = math.sqrt(nslc / 2.0)
+    0.11 / sq  # raises for nslc <= 0, as the reference does
+    try:
+        scan = _lib.load().dpl_ks_critical_distance
+    except (RuntimeError, OSError):  # host arithmetic that needs no library, if slowly (10 ms)
+        return _ks_scan(sq, alpha)
+    return float(scan(int(nslc), float(alpha)))
+
+
+def _ks_scan(sq: float, alpha: float) -> float:
+    cur = 0.01
+    while cur <= 1.0:
+        value = cur * (sq + 0.12 + 0.11 / sq)
+        pvalue = 0
+        for t in range(1, 101):
+            pvalue += ((-1) ** (t - 1)) * math.exp(-2 * (value**2) * (t**2))
+        if max(0.0, min(1.0, 2 * pvalue)) <= alpha:
+            return cur
+        cur += 0.001
+    return 0.1
 
 
 def _method_name(method) -> str:

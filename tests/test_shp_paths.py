@@ -159,3 +159,13 @@ def test_ks_windows_at_the_limit(n, hw):
     want = want.reshape(win.shape[1:])
     want[hw] = False
     np.testing.assert_array_equal(got[r // 3, c // 3], want)
+
+
+def test_ks_critical_distance_without_the_library(monkeypatch, tmp_path):
+    from dolphin_gb300 import _lib
+    from dolphin_gb300.shp import ks_critical_distance
+
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "missing.so")
+    for n, alpha in [(1, 0.05), (20, 0.001), (64, 0.5)]:
+        assert ks_critical_distance(n, alpha) == O.ks_critical_distance(n, alpha)
