@@ -59,7 +59,7 @@ SIGNATURES = {
     "dpl_ps_block": (_i, [_p, _i64, _i64, _f, _i, _d, _i64, _p, _p, _p, _p]),
     "dpl_shp_glrt_workspace_size": (_sz, [_i64, _i64]),
     "dpl_shp_glrt": (_i, [_p, _p, _i64, _i64, _i, _i, _i, _i, _i, _f, _p, _p, _sz, _p]),
-    "dpl_ks_critical_distance": (_d, [_i64, _d]),
+    "dpl_ks_critical_distance": (_d, [_d, _d]),
     "dpl_shp_ks_workspace_size": (_sz, [_i64, _i64, _i64]),
     "dpl_shp_ks": (_i, [_p, _i64, _i64, _i64, _i, _i, _i, _i, _d, _i, _p, _p, _sz, _p]),
     "dpl_phase_link_workspace_size": (_sz, [C.POINTER(PlParams)]),

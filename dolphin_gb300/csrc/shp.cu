@@ -651,8 +651,8 @@ size_t dpl::ks_workspace_size(int64_t nslc, int64_t rows, int64_t cols) {
 // its order, so the distance is the same double: the power of two of `value` through pow()
 // and the terms through exp(), as its interpreter evaluates them.  Host code: as a Python
 // loop the scan took 4-7 ms a call, longer than the kernels.
-extern "C" double dpl_ks_critical_distance(int64_t nslc, double alpha) {
-    const double n_eff = (double)nslc / 2.0, sq = std::sqrt(n_eff);
+extern "C" double dpl_ks_critical_distance(double nslc, double alpha) {
+    const double n_eff = nslc / 2.0, sq = std::sqrt(n_eff);
     double cur = 0.01;
     while (cur <= 1.0) {
         const double value = cur * (sq + 0.12 + 0.11 / sq);

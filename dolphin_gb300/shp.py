@@ -25,7 +25,7 @@ def glrt_threshold(alpha: float) -> float:
     return float(2 * gammaincinv(0.5, 1 - alpha))
 
 
-def ks_critical_distance(nslc: int, alpha: float) -> float:
+def ks_critical_distance(nslc: float, alpha: float) -> float:
     """Critical ECDF distance: the reference's scan (shp/_ks.py:221-239).
 
     Scans distances from 0.01 in steps of 0.001 and returns the first whose
@@ -37,7 +37,7 @@ def ks_critical_distance(nslc: int, alpha: float) -> float:
         scan = _lib.load().dpl_ks_critical_distance
     except (RuntimeError, OSError):  # host arithmetic that needs no library, if slowly (10 ms)
         return _ks_scan(sq, alpha)
-    return float(scan(int(nslc), float(alpha)))
+    return float(scan(float(nslc), float(alpha)))
 
 
 def _ks_scan(sq: float, alpha: float) -> float:

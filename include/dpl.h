@@ -96,8 +96,9 @@ dpl_status dpl_shp_glrt(const float* mean, const float* var, int64_t rows, int64
  * is_shp    : (rows / sy, cols / sx, 2*hy+1, 2*hx+1) uint8 out
  * workspace : dpl_shp_ks_workspace_size(nslc, rows, cols) bytes
  * ------------------------------------------------------------------------------- */
-/* The critical distance itself (host code): the reference's scan, nslc >= 1. */
-double dpl_ks_critical_distance(int64_t nslc, double alpha);
+/* The critical distance itself (host code): the reference's scan, nslc > 0 (not
+ * necessarily whole). */
+double dpl_ks_critical_distance(double nslc, double alpha);
 size_t dpl_shp_ks_workspace_size(int64_t nslc, int64_t rows, int64_t cols);
 dpl_status dpl_shp_ks(const float* amp_stack, int64_t nslc, int64_t rows, int64_t cols, int hy,
                       int hx, int sy, int sx, double cutoff, int is_sorted, uint8_t* is_shp,
