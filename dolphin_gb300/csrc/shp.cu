@@ -690,6 +690,8 @@ extern "C" dpl_status dpl_shp_ks(const float* amp_stack, int64_t nslc, int64_t r
     const int wy = 2 * hy + 1, wx = 2 * hx + 1;
     const int out_rows = (int)(rows / sy), out_cols = (int)(cols / sx);
     if (out_rows == 0 || out_cols == 0) return DPL_OK;
+    if (2 * (n + 1) * sizeof(int) + (size_t)wy * wx * n * sizeof(float) > 200 * 1024)
+        return fail(DPL_ERR_UNSUPPORTED, "dpl_shp_ks: window too large");
     // ECDF tables: T[k] = k-fold float64 sum of 1/n; admissible partner interval per i1
     std::vector<double> T(n + 1, 0.0);
     const double step = 1.0 / n;
@@ -757,8 +759,6 @@ extern "C" dpl_status dpl_shp_ks(const float* amp_stack, int64_t nslc, int64_t r
     const auto bytes_for = [&](int r, int c, int pitch) {
         return region(r, c) * pitch * sizeof(float) + (size_t)r * c * ((wy * wx + 31) / 32) * sizeof(uint32_t);
     };
-    if (2 * (n + 1) * sizeof(int) + region(1, 1) * n * sizeof(float) > 200 * 1024)
-        return fail(DPL_ERR_UNSUPPORTED, "dpl_shp_ks: window too large");
     // an odd pitch (no bank conflicts) wherever one pixel's window has room for it
     a.pitch = bytes_for(1, 1, n | 1) <= 227 * 1024 ? n | 1 : n;
     const auto smem_for = [&](int r, int c) { return bytes_for(r, c, a.pitch); };
