@@ -118,7 +118,8 @@ __device__ __noinline__ bool glrt_test(float s1, float s2, float nslc, float thr
     bool shp = thr > stat;
     // the rounding of the three logarithms and of their cancelling sum
     const float err = nslc * 3e-7f * (fabsf(lp) + fabsf(l1) + fabsf(l2));
-    if (fabsf(stat - thr) <= fmaf(1e-5f, thr, err)) shp = glrt_exact(s1, s2, nslc, thr);
+    // (a scale of 0 has an infinite logarithm and error, and no neighbour)
+    if (s1 > 0.f && s2 > 0.f && fabsf(stat - thr) <= fmaf(1e-5f, thr, err)) shp = glrt_exact(s1, s2, nslc, thr);
     return shp;
 }
 
@@ -255,10 +256,16 @@ __global__ void __launch_bounds__(256, 4) k_glrt(const __grid_constant__ CUtenso
         const int ur0 = in_r - a.hy, uc0 = in_c - a.hx;
         const float s1 = raw[(in_r - rr0) * a.box_w + (in_c - x0)];
         const float* row = raw + (r0 + wa0 - rr0) * a.box_w + (c0 - x0);
-        const float center = a.center * s1, half = a.half * s1, margin = fmaf(5e-7f, center, 1e-40f);
+        // a pixel of scale 0 (no data) or NaN is nobody's neighbour: the statistic is NaN or
+        // infinite.  No column of it is valid and no distance near the interval's end: each
+        // of its tests would else take the double-precision route (1024 x 2048 pixels, a
+        // quarter of them 0: 8.5 ms instead of 0.24).
+        const bool live = s1 > 0.f || a.nslc < 0;  // (a negative count: the statistic is -inf)
+        const float center = a.center * s1, half = a.half * s1;
+        const float margin = live ? fmaf(5e-7f, center, 1e-40f) : -1.f;
         const float k1 = a.four_c * s1;
         // valid window columns v0 .. v1 - 1 and rows of the unclamped origin
-        const int v0 = max(0, -uc0), v1 = min(wx, a.cols - uc0);
+        const int v0 = max(0, -uc0), v1 = live ? min(wx, a.cols - uc0) : 0;
         const auto columns = [&](int b0, int nb) {
             const int lo = max(v0 - b0, 0), hi = min(v1 - b0, nb);
             return hi > lo ? (0xffffffffu >> (32 - (hi - lo))) << lo : 0u;
