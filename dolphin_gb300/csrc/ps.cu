@@ -6,12 +6,15 @@
 // sums along axis 0, NaN entries replaced by 0, divisions by the count rounded
 // once, no FMA contraction.  4N bytes in, 9 bytes out.
 //
-// Bound by HBM with the loads in flight: 2048 x 4096 pixels at N = 30 take 155 us (7.0 TB/s,
-// part of it from L2);
-// with the NaN bookkeeping on every sample, issue-bound, they took 386 us.
-// A pixel whose plain sum is a number has no NaN, so the replacement, its bookkeeping and
-// the count run only where that sum is NaN; all loads are issued before the first sum.
-// (Two or four pixels per thread, for wider loads, were slower at every size.)
+// Bound by HBM with the loads in flight: 2048 x 4096 pixels at N = 30 take 155 us (7.0
+// TB/s, part of it from L2).  A pixel whose plain sum is a number has no NaN, so the
+// replacement, its bookkeeping and the count run only where that sum is NaN (on every
+// sample, issue-bound, 386 us); all loads are issued before the first sum.  A pixel with
+// a NaN reads its samples again, eight loads in flight: with 1 % of the samples NaN, so
+// that every warp takes both routes, the call takes 347 us where it takes 219 without
+// NaNs (487 one load after the other).  Keeping that route's samples in registers as
+// well took 280, but 2 to 20 % longer without NaNs.  Two or four pixels per thread, for
+// wider loads, were slower at every size.
 #include "dpl_common.cuh"
 
 namespace dpl {
@@ -40,12 +43,12 @@ struct PsOut {
     }
 };
 
-// any n: NaN samples replaced by 0 and left out of the count; x(t) gives sample t
+// any n: NaN samples replaced by 0 and left out of the count; x(t) loads sample t
 template <class Sample>
 __device__ __forceinline__ void ps_pixel(Sample&& x, int n, int64_t p, const PsOut& out) {
     float sum = 0.f;
     int cnt = 0;
-#pragma unroll 1
+#pragma unroll 8
     for (int t = 0; t < n; ++t) {
         const float v = x(t);
         const bool nan = isnan(v);
@@ -55,7 +58,7 @@ __device__ __forceinline__ void ps_pixel(Sample&& x, int n, int64_t p, const PsO
     }
     const float mean = fdiv(sum, (float)cnt);
     float ss = 0.f;
-#pragma unroll 1
+#pragma unroll 8
     for (int t = 0; t < n; ++t) {
         const float v = x(t);
         const float d = isnan(v) ? 0.f : fsub(v, mean);
