@@ -620,8 +620,8 @@ static dpl_status launch_post(const PostArgs& q, int64_t npix, cudaStream_t s) {
 // ---------------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------------
-static void fill_pix_layout(PixArgs& a, int n, int wx, bool lu = false) {
-    PixLayout L = make_layout(n, wx, lu);
+static void fill_pix_layout(PixArgs& a, int n, int wx, bool lu = false, bool inverse = false) {
+    PixLayout L = make_layout(n, wx, lu, inverse);
     a.n = n;
     a.np = L.np;
     a.stg = L.stg;
@@ -767,7 +767,7 @@ static dpl_status launch_pixel(PixArgs& a, cudaStream_t s, int* fb = nullptr, in
     dpl_status st = MODE == kSolveOnly && a.n <= 64 ? launch_solve_reg(a, s) : launch_pixel_pass<MODE, false>(a, s);
     if (st != DPL_OK) return st;
     PixArgs b = a;
-    fill_pix_layout(b, a.n, 2 * a.hx + 1, true);
+    fill_pix_layout(b, a.n, 2 * a.hx + 1, true, a.nc_list != nullptr);
     b.list = a.fb_list;
     b.list_count = a.fb_count;
     st = launch_pixel_pass<MODE, true>(b, s);
@@ -776,6 +776,7 @@ static dpl_status launch_pixel(PixArgs& a, cudaStream_t s, int* fb = nullptr, in
     a.redo_list = fb + 64;
     st = launch_eigh(a, s);
     if (st != DPL_OK) return st;
+    fill_pix_layout(b, a.n, 2 * a.hx + 1, true);
     b.list = a.redo_list;
     b.list_count = a.redo_count;
     b.nc_list = nullptr;  // every step, nothing listed

@@ -12,16 +12,16 @@ namespace dpl {
 // ---------------------------------------------------------------------------------
 // k_pixel: per-warp shared-memory layout
 // ---------------------------------------------------------------------------------
-// C (packed complex) | W1 (packed real) | S: staging for the window rows, or R (packed
-// complex) + W2 (packed real), or the full n x n LU of the fallback | v | d | piv
 struct PixLayout {
     int n, np, stg, ldg;
     size_t off_C, off_G, off_S, off_v, off_d, off_piv, bytes;
 };
 
 // C (packed complex) | G (n x ldg real) | S: staging for the covariance's window rows,
-// or R (packed complex), or the full n x n LU of the LU pass and its inverse | v | d | piv
-inline PixLayout make_layout(int n, int wx, bool lu) {
+// or R (packed complex), or the full n x n LU of the LU pass, with its inverse where
+// that pass looks for pixels far from the stopping rule (s_lu_stalls; elsewhere it would
+// cost resident warps: 6 -> 4 per CTA at N = 30) | v | d | piv
+inline PixLayout make_layout(int n, int wx, bool lu, bool inverse = false) {
     PixLayout L{};
     const size_t T = (size_t)n * (n + 1) / 2;
     L.n = n;
@@ -37,7 +37,7 @@ inline PixLayout make_layout(int n, int wx, bool lu) {
     L.off_C = take(T * sizeof(cfloat));
     L.off_G = take((size_t)n * L.ldg * sizeof(float));
     size_t s_bytes = std::max((size_t)L.stg * sizeof(cfloat), T * sizeof(cfloat));
-    if (lu) s_bytes = std::max(s_bytes, (size_t)n * (n + (n | 1)) * sizeof(cfloat));  // LU, explicit inverse
+    if (lu) s_bytes = std::max(s_bytes, (size_t)n * (n + (inverse ? n | 1 : 0)) * sizeof(cfloat));
     L.off_S = take(s_bytes);
     L.off_v = take(64 * sizeof(cfloat));
     L.off_d = take(64 * sizeof(float));
