@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(256) k_pixel(PixArgs a) {
     unsigned char* base = pix_smem + warp * a.warp_bytes;
     SolveMats m;
     m.C = reinterpret_cast<cfloat*>(base + a.off_C);
+    m.M = m.C + tri(a.n) - a.n * a.ldg;
     m.G = reinterpret_cast<float*>(base + a.off_G);
     m.ldg = a.ldg;
     m.R = reinterpret_cast<cfloat*>(base + a.off_S);
@@ -253,16 +254,24 @@ __global__ void __launch_bounds__(256) k_pixel(PixArgs a) {
     const int64_t total = a.list ? (int64_t)*a.list_count : a.npix;
     for (int64_t idx = (int64_t)blockIdx.x * nwarps + warp; idx < total; idx += (int64_t)gridDim.x * nwarps) {
         const int64_t p = a.list ? (int64_t)a.list[idx] : idx;
-        if (MODE == kSolveOnly) {
+        const auto load = [&]() {  // the pixel's matrix into m.C, where it is not formed here
+            if (MODE != kSolveOnly) return;
             __syncwarp();
             if (a.Cplanar) {
                 // unnormalised planar sums: C_ij = numer_ij r_i r_j, r = 1 / sqrt(amp), 0 where
                 // r_i r_j >= 1e6 (covariance.py:131-142)
                 const float* src = a.Cplanar + p * n * n;
+                float* rv = m.d;
+                for (int i = lane; i < n; i += 32) rv[i] = __frsqrt_rn(src[i]);
+                __syncwarp();
+#pragma unroll 4
                 for (int i = 0; i < n; ++i) {
-                    const float ri = __frsqrt_rn(src[i]);
-                    for (int j = lane; j <= i; j += 32) {
-                        const float f = ri * __frsqrt_rn(src[j]);
+                    const float ri = rv[i];
+#pragma unroll
+                    for (int q = 0; q < NB; ++q) {
+                        const int j = lane + 32 * q;
+                        if (j > i) continue;
+                        const float f = ri * rv[j];
                         const bool ok = f < 1e6f;
                         const int o = i * (i - 1) / 2 + j;  // pair (i, j), i > j
                         m.C[pk(i, j)] = i == j ? cmake(ok ? src[i] * f : 0.f, 0.f)
@@ -276,7 +285,8 @@ __global__ void __launch_bounds__(256) k_pixel(PixArgs a) {
                     for (int j = lane; j <= i; j += 32) m.C[pk(i, j)] = src[i * n + j];
             }
             __syncwarp();
-        } else {
+        };
+        if (MODE != kSolveOnly) {
             int count = 0;
             warp_covariance<NB>(a, p, m.C, m.R, m.d, lane, &count);
             if (a.counts && lane == 0) a.counts[p] = count;
@@ -287,7 +297,7 @@ __global__ void __launch_bounds__(256) k_pixel(PixArgs a) {
                 for (int j = lane; j < n; j += 32) dst[i * n + j] = cget(m.C, i, j);
             __syncwarp();
         } else {
-            solve_pixel<NB, kLU>(a, p, m, lane);
+            solve_pixel<NB, kLU>(a, p, m, lane, load);
         }
     }
 }
@@ -666,6 +676,19 @@ template <int MODE, bool kLU>
 static dpl_status launch_pixel_pass(const PixArgs& a, cudaStream_t s) {
     // as many warps per CTA as fit ~100 KB (two CTAs per SM), at most 8
     int warps = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(100 * 1024) / a.warp_bytes));
+    if (kLU && a.nc_list) {
+        // with the inverse a warp takes a quarter more, and shared memory bounds the resident
+        // warps: the CTA size that leaves the most (228 KB per SM, 1 KB of them the system's
+        // per CTA; registers allow 32)
+        int most = 0;
+        for (int w = warps; w >= 1; --w) {
+            const int resident = std::min(32, w * (int)((228 * 1024) / (w * a.warp_bytes + 1024)));
+            if (resident > most) {
+                most = resident;
+                warps = w;
+            }
+        }
+    }
     size_t smem = (size_t)warps * a.warp_bytes;
     if (smem > 220 * 1024) return fail(DPL_ERR_UNSUPPORTED, "per-pixel shared memory exceeds the SM limit");
     int dev = 0, sms = 0;
@@ -767,7 +790,8 @@ static dpl_status launch_pixel(PixArgs& a, cudaStream_t s, int* fb = nullptr, in
     dpl_status st = MODE == kSolveOnly && a.n <= 64 ? launch_solve_reg(a, s) : launch_pixel_pass<MODE, false>(a, s);
     if (st != DPL_OK) return st;
     PixArgs b = a;
-    fill_pix_layout(b, a.n, 2 * a.hx + 1, true, a.nc_list != nullptr);
+    const int wx = MODE == kSolveOnly ? 1 : 2 * a.hx + 1;  // no window rows are staged where C is given
+    fill_pix_layout(b, a.n, wx, true, a.nc_list != nullptr);
     b.list = a.fb_list;
     b.list_count = a.fb_count;
     st = launch_pixel_pass<MODE, true>(b, s);
@@ -776,7 +800,7 @@ static dpl_status launch_pixel(PixArgs& a, cudaStream_t s, int* fb = nullptr, in
     a.redo_list = fb + 64;
     st = launch_eigh(a, s);
     if (st != DPL_OK) return st;
-    fill_pix_layout(b, a.n, 2 * a.hx + 1, true);
+    fill_pix_layout(b, a.n, wx, true);
     b.list = a.redo_list;
     b.list_count = a.redo_count;
     b.nc_list = nullptr;  // every step, nothing listed

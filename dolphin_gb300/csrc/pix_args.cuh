@@ -18,9 +18,10 @@ struct PixLayout {
 };
 
 // C (packed complex) | G (n x ldg real) | S: staging for the covariance's window rows,
-// or R (packed complex), or the full n x n LU of the LU pass, with its inverse where
-// that pass looks for pixels far from the stopping rule (s_lu_stalls; elsewhere it would
-// cost resident warps: 6 -> 4 per CTA at N = 30) | v | d | piv
+// or R (packed complex), or the full n x n LU of the LU pass | v | d | piv.  With `inverse`
+// there is room before C for what the inverse of s_lu_stalls needs beyond C's own (it
+// ends where C ends, and C is loaded again after it): only where the LU pass looks for
+// pixels far from the stopping rule, because it costs resident warps.
 inline PixLayout make_layout(int n, int wx, bool lu, bool inverse = false) {
     PixLayout L{};
     const size_t T = (size_t)n * (n + 1) / 2;
@@ -34,10 +35,11 @@ inline PixLayout make_layout(int n, int wx, bool lu, bool inverse = false) {
         o = align_up(o + bytes, 16);
         return at;
     };
+    if (inverse) take(((size_t)n * L.ldg - T) * sizeof(cfloat));
     L.off_C = take(T * sizeof(cfloat));
     L.off_G = take((size_t)n * L.ldg * sizeof(float));
     size_t s_bytes = std::max((size_t)L.stg * sizeof(cfloat), T * sizeof(cfloat));
-    if (lu) s_bytes = std::max(s_bytes, (size_t)n * (n + (inverse ? n | 1 : 0)) * sizeof(cfloat));
+    if (lu) s_bytes = std::max(s_bytes, (size_t)n * n * sizeof(cfloat));
     L.off_S = take(s_bytes);
     L.off_v = take(64 * sizeof(cfloat));
     L.off_d = take(64 * sizeof(float));

@@ -37,6 +37,7 @@ __device__ __forceinline__ cfloat cget(const cfloat* C, int i, int j) {
 
 struct SolveMats {
     cfloat* C;   // packed coherence
+    cfloat* M;   // n x ldg, over C's end: the explicit inverse of the LU pass's probe
     float* G;    // n x ldg real work matrix
     int ldg;
     cfloat* R;   // packed complex (EMI factor, or C o |C| for EVD); full n x n LU in the LU pass
@@ -384,19 +385,23 @@ __device__ bool s_iterate(cfloat (&v)[NB], Op&& op) {
     return !(diff > 1e-5f);  // a NaN difference ends the loop too, as in the reference
 }
 
-// Full solve for one pixel whose packed coherence matrix is in m.C.  With kLU the
+// Full solve for one pixel whose packed coherence matrix load() puts into m.C.  With kLU the
 // EMI step uses LU with partial pivoting; otherwise a pixel whose shifted matrix is
 // not positive definite is appended to a.fb_list and left for the LU pass.
-template <int NB, bool kLU>
-__device__ void solve_pixel(const PixArgs& a, int64_t p, const SolveMats& m, int lane) {
+template <int NB, bool kLU, class Load>
+__device__ void solve_pixel(const PixArgs& a, int64_t p, const SolveMats& m, int lane, Load&& load) {
     const int n = a.n, ld = m.ldg;
     cfloat* C = m.C;
     float* G = m.G;
-    if (a.baseline_lag > 0) {
-        for (int i = a.baseline_lag; i < n; ++i)
-            for (int j = lane; j <= i - a.baseline_lag; j += 32) C[pk(i, j)] = cmake(0.f, 0.f);
-        __syncwarp();
-    }
+    auto reload = [&]() {
+        load();
+        if (a.baseline_lag > 0) {
+            for (int i = a.baseline_lag; i < n; ++i)
+                for (int j = lane; j <= i - a.baseline_lag; j += 32) C[pk(i, j)] = cmake(0.f, 0.f);
+            __syncwarp();
+        }
+    };
+    reload();
     if (a.closure) {
         for (int i = lane; i < n - 2; i += 32) {
             const cfloat c = cmulc(cmul(cget(C, i, i + 1), cget(C, i + 1, i + 2)), cget(C, i, i + 2));
@@ -484,8 +489,15 @@ __device__ void solve_pixel(const PixArgs& a, int64_t p, const SolveMats& m, int
             // pixels use all 49 steps, 1.4 M of the pass's 1.65 M cycles at N = 30 (the pass
             // on 1034 x 1046 pixels: 806 -> 353 us; at N = 10 on 128 x 128: 156 -> 60 us)
             // (it takes over all but those whose |Gamma| is not positive definite in double:
-            // these come back in a pass of their own, which iterates)
-            stalled = a.nc_list && s_lu_stalls<NB>(A, n, src, A + n * n, m.v, lane);
+            // these come back in a pass of their own, which iterates).  Where every pixel is
+            // listed (a large beta; 300 x 320 pixels) the whole call goes from 9.2 to 6.0 ms at
+            // N = 12, 32.1 to 29.2 at 30 and 164 to 112 at 45, but from 13.8 to 16.4 at N = 21:
+            // there most pixels come to the rule and the probe's memory costs resident warps
+            // (18 to 23: 1 to 18 %).
+            if (a.nc_list) {
+                stalled = s_lu_stalls<NB>(A, n, src, m.M, m.v, lane);
+                reload();
+            }
             converged = !stalled && s_iterate<NB>(v, [&](cfloat(&x)[NB]) { s_lu_solve<NB>(A, n, src, x, lane); });
             s_publish<NB>(m.v, v, n, lane);
             float s = 0.f;

@@ -1,5 +1,6 @@
-"""Shared memory of a warp of the LU pass: the n x n matrix, and room for its explicit
-inverse only where the pass is asked for it (host code, compiled here)."""
+"""Shared memory of a warp of the LU pass: the n x n matrix, and only where the pass is
+asked for its explicit inverse, room for the part of that which C does not hold (host
+code, compiled here)."""
 
 import shutil
 import subprocess
@@ -15,7 +16,9 @@ PROGRAM = """
 #include "pix_args.cuh"
 int main() {
     for (int n : {%s})
-        for (int wx : {1, 23}) printf("%%d %%d %%zu\\n", n, wx, dpl::make_layout(n, wx, true).bytes);
+        for (int wx : {1, 23})
+            printf("%%d %%d %%zu %%zu\\n", n, wx, dpl::make_layout(n, wx, true).bytes,
+                   dpl::make_layout(n, wx, true, true).bytes);
 }
 """
 
@@ -24,7 +27,7 @@ def _up(x, a):
     return -(-x // a) * a
 
 
-def test_lu_pass_without_inverse(tmp_path):
+def test_lu_pass(tmp_path):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not Path(nvcc).exists():
         pytest.skip("needs nvcc")
@@ -35,7 +38,9 @@ def test_lu_pass_without_inverse(tmp_path):
                     str(ROOT / "dolphin_gb300" / "csrc"), "-o", str(exe), str(src)], check=True)
     lines = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split("\n")
     for line in filter(None, lines):
-        n, wx, got = map(int, line.split())
+        n, wx, got, probing = map(int, line.split())
         tri = n * (n + 1) // 2
         parts = [8 * tri, 4 * n * (n | 1), 8 * max(wx * ((n + 1) & ~1) + 32, tri, n * n), 8 * 64, 4 * 64, 4 * 128]
         assert got == _up(sum(_up(p, 16) for p in parts), 128), (n, wx)
+        # the inverse, n x (n | 1), lies over C's end
+        assert probing == _up(sum(_up(p, 16) for p in [8 * (n * (n | 1) - tri)] + parts), 128), (n, wx)
