@@ -230,6 +230,81 @@ __device__ void warp_covariance(const PixArgs& a, int64_t p, cfloat* C, cfloat* 
     if (count_out) *count_out = count;
 }
 
+// Makes a normalised packed matrix of k_cov_simt what warp_covariance gives, bit for bit:
+// the imaginary rounding residues of the diagonal, which the planar layout has no room for,
+// and above n = 32 the imaginary parts of the rows 32 .. n - 1 by the columns 0 .. 31, which
+// warp_covariance sums for the pairs the other way round, rounding the other product.
+template <int NB>
+__device__ void warp_residues(const PixArgs& a, int64_t p, cfloat* C, cfloat* stg, float* amp, int lane) {
+    const int n = a.n, wy = 2 * a.hy + 1, wx = 2 * a.hx + 1, np = a.np;
+    const int out_r = (int)(p / a.out_cols), out_c = (int)(p - (int64_t)out_r * a.out_cols);
+    const int r0 = clamp_start_i(a.sy / 2 + out_r * a.sy, a.hy, wy, a.rows);
+    const int c0 = clamp_start_i(a.sx / 2 + out_c * a.sx, a.hx, wx, a.cols);
+    float sum[NB], im[NB];  // of rows lane, 32 + lane: |z|^2 and its residue
+    float aim[NB == 2 ? 32 : 1];  // pairs (lane, 32 + j)
+#pragma unroll
+    for (int q = 0; q < NB; ++q) sum[q] = im[q] = 0.f;
+#pragma unroll
+    for (int j = 0; j < (NB == 2 ? 32 : 1); ++j) aim[j] = 0.f;
+    const auto diagonal = [&](int q, cfloat z) {
+        sum[q] = fadd(sum[q], fmaf(z.re, z.re, fmul(z.im, z.im)));
+        im[q] = fadd(im[q], fmaf(z.im, z.re, -fmul(z.re, z.im)));
+    };
+    for (int wa = 0; wa < wy; ++wa) {
+        const uint64_t rm = row_mask(a, p, wa, wx, lane);
+        if (rm == 0ull) continue;
+        const cfloat* src = a.zt + ((int64_t)(r0 + wa) * a.cols + c0) * n;
+        if constexpr (NB == 1) {
+            const int t = lane < n ? lane : 0;
+#pragma unroll 8
+            for (int wb = 0; wb < wx; ++wb) {
+                const cfloat z = src[wb * n + t];
+                if ((rm >> wb) & 1ull) diagonal(0, z);
+            }
+        } else {
+            __syncwarp();
+            for (int idx = lane; idx < a.stg; idx += 32) {
+                const int b = idx / np, t = idx - b * np;
+                stg[idx] = (b < wx && t < n) ? src[b * n + t] : cmake(0.f, 0.f);
+            }
+            __syncwarp();
+            for (int wb = 0; wb < wx; ++wb) {
+                if (!((rm >> wb) & 1ull)) continue;
+                const cfloat* s = stg + wb * np;
+                const cfloat z = s[lane];
+                diagonal(0, z);
+                diagonal(1, s[32 + lane]);
+                const float4* sj = reinterpret_cast<const float4*>(s + 32);
+#pragma unroll
+                for (int j2 = 0; j2 < 16; ++j2) {
+                    const float4 q = sj[j2];
+                    aim[2 * j2] = fadd(aim[2 * j2], fmaf(z.im, q.x, -fmul(z.re, q.y)));
+                    aim[2 * j2 + 1] = fadd(aim[2 * j2 + 1], fmaf(z.im, q.z, -fmul(z.re, q.w)));
+                }
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NB; ++q) amp[32 * q + lane] = sum[q];
+    __syncwarp();
+    const auto normalised = [&](float x, int i, int j) {
+        const float s = fsqrt(fmul(amp[i], amp[j]));
+        return s > 1e-6f ? fdiv(x, s) : 0.f;
+    };
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int i = lane + 32 * q;
+        if (i < n) C[pk(i, i)].im = normalised(im[q], i, i);
+    }
+    if constexpr (NB == 2) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if (32 + j < n) C[pk(32 + j, lane)].im = normalised(-aim[j], 32 + j, lane);
+    }
+    __syncwarp();
+}
+
 }  // namespace dpl
 
 #include "cov_simt.cuh"
@@ -257,7 +332,21 @@ __global__ void __launch_bounds__(256) k_pixel(PixArgs a) {
         const auto load = [&]() {  // the pixel's matrix into m.C, where it is not formed here
             if (MODE != kSolveOnly) return;
             __syncwarp();
-            if (a.Cplanar) {
+            if (a.Cplanar && a.planar_norm) {
+                const float* src = a.Cplanar + p * n * n;
+#pragma unroll 4
+                for (int i = 0; i < n; ++i) {
+#pragma unroll
+                    for (int q = 0; q < NB; ++q) {
+                        const int j = lane + 32 * q;
+                        if (j > i) continue;
+                        const float* z = src + (i == j ? i : n + i * (i - 1) + 2 * j);
+                        m.C[pk(i, j)] = cmake(z[0], i == j ? 0.f : z[1]);
+                    }
+                }
+                __syncwarp();
+                warp_residues<NB>(a, p, m.C, m.R, m.d, lane);
+            } else if (a.Cplanar) {
                 // unnormalised planar sums: C_ij = numer_ij r_i r_j, r = 1 / sqrt(amp), 0 where
                 // r_i r_j >= 1e6 (covariance.py:131-142)
                 const float* src = a.Cplanar + p * n * n;
@@ -1160,14 +1249,19 @@ static dpl_status pl_finish(PlState& S, cudaStream_t s, bool cov_done) {
         st = timed(s, 1, [&] {
             return launch_pixel<kSolveOnly>(a, s, w.fb, P.nonconverged_mode == 0 ? w.nc : nullptr);
         });
-    } else if (w.Cg) {
+    } else if (w.Cg && (P.use_evd || (2 * P.hy + 1) * (2 * P.hx + 1) > n)) {
         // window or strides too large for the tensor-core tiles: float32 covariance on the
         // CUDA cores and the register solver on it, its last iterate kept as in the plain
         // form.  Its explicit inverses cost accuracy where a pixel is ill-conditioned: those
-        // few pixels, and the undecided ones (|Gamma| not positive definite), are listed and
-        // solved by the plain form, then the LU pass takes what both listed.
-        // 512 x 384 outputs, strides 3 x 6, 11 x 23 window, N = 21: 21.1 -> 5.9 ms on the device
-        // (the fused k_pixel took 20.6 ms; k_cov_simt 3.6, k_solve_reg 1.5, the list 0.3).
+        // pixels, and the undecided ones (|Gamma| not positive definite), are listed and
+        // solved by the plain form's solver on the same matrices, then the LU pass takes what
+        // that listed.
+        // 512 x 384 outputs, strides 3 x 6, 11 x 23 window, N = 21: 20.6 -> 5.0 ms on the device
+        // against the fused k_pixel.  Few pixels are listed there; where all are (coherence
+        // 0.99, 200 x 150 outputs): N = 21 3.3 -> 1.8 ms, N = 45 22.4 -> 16.8 ms, N = 64 42.2 ->
+        // 35.2 ms.  A window of no more samples than dates lists every pixel for a covariance
+        // that costs next to nothing: N = 30, 15 or 25 samples, is 13 % slower this way than
+        // fused, 45 samples 40 % faster (N = 50: 45 samples 5 % slower, 63 39 % faster).
         st = timed(s, 0, [&] { return launch_cov_simt<1>(cov_simt_block(n), a, w.Cg, s); });
         if (st != DPL_OK) return st;
         st = timed(s, 1, [&]() -> dpl_status {
@@ -1183,15 +1277,18 @@ static dpl_status pl_finish(PlState& S, cudaStream_t s, bool cov_done) {
             b.ill_list = w.nc + 64;
             dpl_status e = launch_solve_reg(b, s);
             if (e != DPL_OK) return e;
-            PixArgs c = a;
+            // the listed pixels from the same matrices
+            PixArgs c = b;
+            const int wx = n > 32 ? 2 * P.hx + 1 : 1;  // window rows are staged above 32 only
+            fill_pix_layout(c, n, wx);
             c.list = b.ill_list;
             c.list_count = b.ill_count;
-            e = launch_pixel_pass<kFused, false>(c, s);
+            e = launch_pixel_pass<kSolveOnly, false>(c, s);
             if (e != DPL_OK) return e;
-            fill_pix_layout(c, n, 2 * P.hx + 1, true);
+            fill_pix_layout(c, n, wx, true);
             c.list = a.fb_list;
             c.list_count = a.fb_count;
-            return launch_pixel_pass<kFused, true>(c, s);
+            return launch_pixel_pass<kSolveOnly, true>(c, s);
         });
     } else {
         // plain form: SIMT covariance fused with the solver
