@@ -1249,7 +1249,7 @@ static dpl_status pl_finish(PlState& S, cudaStream_t s, bool cov_done) {
         st = timed(s, 1, [&] {
             return launch_pixel<kSolveOnly>(a, s, w.fb, P.nonconverged_mode == 0 ? w.nc : nullptr);
         });
-    } else if (w.Cg && (P.use_evd || (2 * P.hy + 1) * (2 * P.hx + 1) > n)) {
+    } else if (w.Cg && ((P.use_evd && !P.compute_crlb) || (2 * P.hy + 1) * (2 * P.hx + 1) > n)) {
         // window or strides too large for the tensor-core tiles: float32 covariance on the
         // CUDA cores and the register solver on it, its last iterate kept as in the plain
         // form.  Its explicit inverses cost accuracy where a pixel is ill-conditioned: those

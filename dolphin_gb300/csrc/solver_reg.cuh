@@ -105,6 +105,16 @@ struct Grp {
         sync();
         return r;
     }
+    __device__ __forceinline__ float max(float v) const {
+#pragma unroll
+        for (int o = (G <= 32 ? G >> 1 : 16); o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(mask, v, o));
+        if (G <= 32) return v;
+        if (lane == 0) x[wig] = v;
+        sync();
+        const float r = fmaxf(x[0], x[1]);
+        sync();
+        return r;
+    }
     __device__ __forceinline__ bool any(bool v) const {
         if (G <= 32) return __any_sync(mask, v);
         v = warp_any(v);
@@ -135,13 +145,22 @@ __device__ __forceinline__ float frcp_nr(float p) {
     return fmaf(r, fmaf(-p, r, 1.f), r);
 }
 
+// A power of two that takes the largest diagonal entry `top` of a positive definite matrix,
+// and so every pivot of its sweep, to 1 or below (1 where it is there already).
+__device__ __forceinline__ float r_scale(float top) {
+    return top > 1.f && top < 1e30f ? __uint_as_float((253u - (__float_as_uint(top) >> 23)) << 23) : 1.f;
+}
+
 // The sweeps broadcast the pivot column through `buf`, two halves used alternately so
 // that one barrier per step suffices: step k writes half k & 1, whose readers (step
 // k - 2) all passed step k - 1's barrier before this thread did.
 
 // Real symmetric sweep of the matrix whose row `gl` is g; on success g holds row `gl` of
-// -A^{-1}.  Returns false (uniformly) if any pivot was <= 0 (the remaining steps then run
-// on meaningless values, without branching).  buf: 2 * KB floats.
+// -A^{-1}.  Row k's 1 - 1/p loses p units of the last place where p > 1 (the CRLB's Fisher
+// matrix, the shifted EMI matrix of a coherent pixel): the strided route, which stands in
+// for a solver without that loss, scales them to pivots of 1 or below.  Returns false
+// (uniformly) if any pivot was <= 0 (the remaining steps then run on meaningless values,
+// without branching).  buf: 2 * KB floats.
 template <int K, int G>
 __device__ __forceinline__ bool r_sweep(f2 (&g)[K / 2], float* buf, const Grp<G>& gr) {
     constexpr int KB = RegShape<K, G>::KB;
@@ -388,8 +407,10 @@ __device__ __forceinline__ float r_iterate(cfloat& v, const Grp<G>& gr, int& ste
 // Full solve for one pixel whose Hermitian coherence matrix is in the planes Cr, Ci (both
 // triangles) and whose |Gamma| is in Gs off the diagonal.  A pixel whose shifted EMI
 // matrix is not positive definite is listed and left for the LU pass (or the plain form).
-// `fetch` loads the group's next pixel.
-template <int K, int G, class Fetch>
+// `fetch` loads the group's next pixel.  kScale: the matrices are scaled (r_sweep), as every
+// launch with an ill_list is; that list is looked up at run time in all instances, because
+// the others compile to slower code without it (N = 30 by 1 %, N = 44 by 5 %).
+template <int K, int G, bool kScale, class Fetch>
 __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, float* Cr, float* Ci, float* Gs, float* U,
                                                 const uint16_t* ptab, const Grp<G>& gr, Fetch&& fetch) {
     using S = RegShape<K, G>;
@@ -410,7 +431,7 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
     const int ref = a.crlb_ref;
     bool inv_nan = true;
     bool crlb_ok = false;
-    float dg = 0.f;
+    float dg = 0.f, unscale = 1.f;
     if (!(a.use_evd && !a.compute_crlb)) {
         // |Gamma| + 1e-6 I -> -|Gamma|^{-1} (round 0), then the CRLB's Fisher matrix
         // FIM = 2L (Gamma o Gamma^{-1} - I), row/col `ref` -> identity, + 1e-6 I (round 1).
@@ -461,6 +482,7 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
                 if (a.compute_crlb) Gi[ref] = 0.f;
             }
             const f2 ff = f2_pack(f, f), minus = f2_pack(-1.f, -1.f);
+            float fd = 0.f;  // the diagonal entry
 #pragma unroll
             for (int q = 0; q < K / 2; ++q) {
                 const f2 ginv = f2_mul(g[q], minus);
@@ -475,12 +497,21 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
                 if (me == 2 * q) x0 = fadd(x0, dadd);
                 if (me == 2 * q + 1) x1 = fadd(x1, dadd);
                 g[q] = f2_pack(x0, x1);
+                if (me == 2 * q) fd = x0;
+                if (me == 2 * q + 1) fd = x1;
             }
             if (!a.compute_crlb) break;
+            if constexpr (kScale) {  // see r_sweep: pivots of 1 or below
+                unscale = r_scale(gr.max(fd));
+                const f2 c = f2_pack(unscale, unscale);
+#pragma unroll
+                for (int q = 0; q < K / 2; ++q) g[q] = f2_mul(g[q], c);
+            }
         }
     }
     const bool evd = a.use_evd || inv_nan;
-    if (row) a.crlb[p * n + me] = !a.compute_crlb || me == ref ? 0.f : (crlb_ok ? sqrtf(-dg) : nanf(""));
+    const float var = kScale ? -dg * unscale : -dg;
+    if (row) a.crlb[p * n + me] = !a.compute_crlb || me == ref ? 0.f : (crlb_ok ? sqrtf(var) : nanf(""));
 
     // One matrix (re, im) and one iteration for both estimators, the matrix formed as
     // C o Gs: EMI iterates with -(A - 0.99 I)^{-1} (the negated sweep result), its
@@ -514,6 +545,15 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
         im[q] = f2_mul(f2_ld(ci, q), gq);
     }
     if (!evd) {
+        if constexpr (kScale) {  // see r_sweep: pivots of 1 or below (the iterates are normalised)
+            const float top = gr.max(act ? Gi[me] : 0.f), scale = r_scale(top);
+            const f2 c = f2_pack(scale, scale);
+#pragma unroll
+            for (int q = 0; q < K / 2; ++q) {
+                re[q] = f2_mul(re[q], c);
+                im[q] = f2_mul(im[q], c);
+            }
+        }
         if (act) {
             Gi[me] = gd;
             cr[me] = cd;
@@ -550,12 +590,13 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
         diff = r_iterate<G>(v, gr, steps, op);
     }
     // ill-conditioned for the explicit inverses, or not decided by them: listed for the
-    // plain form.  Of 160 k pixels at N = 45 (11 x 23 windows over parcels of different
-    // coherence) every phase that came out more than 1e-4 rad from the plain form's had a
-    // diagonal entry of |Gamma|^{-1} above 50 or more than 45 steps; 0.1 % are listed.
-    if (a.ill_list && !a.use_evd) {
+    // plain form's solver.  The others' errors against FP64 are the plain form's: over N = 5 to
+    // 64, windows of 63 to 253 samples, decaying, coherent (0.8 to 0.99) and EVD scenes the
+    // root mean squares of the CRLB agree to 4 % and those of the phases to 5 % or, near the
+    // last place (2e-7 rad), 11 %; no phase comes out more than 1e-4 rad worse.
+    if (a.ill_list && (!a.use_evd || a.compute_crlb)) {
         const bool ill = gr.any(row && gd > 32.f);
-        if ((evd || ill || steps > 24) && me == 0) a.ill_list[atomicAdd(a.ill_count, 1)] = (int)p;
+        if ((inv_nan || ill || (!evd && steps > 24)) && me == 0) a.ill_list[atomicAdd(a.ill_count, 1)] = (int)p;
     }
     // 49 steps without meeting the stopping rule (a NaN difference stops the loop, as in
     // the reference): listed for the dense eigensolver
@@ -652,7 +693,7 @@ __device__ __forceinline__ void solve_pixel_reg(const PixArgs& a, int64_t p, flo
 // of which the lower triangle is read.
 // Two CTAs per SM (128 registers) wherever two CTAs' shared memory fits, K <= 46: the
 // two-warp instances would take more registers and one CTA.
-template <int K, int G>
+template <int K, int G, bool kScale>
 __global__ void __launch_bounds__(256, (G == 64 && K > 46) ? 1 : 2) k_solve_reg(PixArgs a) {
     using S = RegShape<K, G>;
     constexpr int LD = S::LD;
@@ -750,7 +791,7 @@ __global__ void __launch_bounds__(256, (G == 64 && K > 46) ? 1 : 2) k_solve_reg(
         }
         gr.sync();
         const int64_t next = p + stride;
-        solve_pixel_reg<K, G>(a, p, Cr, Ci, Gs, U, ptab, gr, [&]() {
+        solve_pixel_reg<K, G, kScale>(a, p, Cr, Ci, Gs, U, ptab, gr, [&]() {
             in.load(a, next < a.npix ? next : p, ptab, me);  // unconditional: the old values die here
         });
     }
@@ -758,8 +799,8 @@ __global__ void __launch_bounds__(256, (G == 64 && K > 46) ? 1 : 2) k_solve_reg(
 
 // Host launch of the instance with K slots and G threads per pixel: 8 warps per CTA,
 // 256 / G pixel groups; a persistent grid of at most 8 waves.
-template <int K, int G>
-dpl_status launch_solve_reg_k(const PixArgs& a, cudaStream_t s) {
+template <int K, int G, bool kScale>
+dpl_status launch_solve_reg_kl(const PixArgs& a, cudaStream_t s) {
     const int warps = 8;
     const int groups = warps * 32 / G;
     const size_t smem = (size_t)groups * RegShape<K, G>::FLOATS * sizeof(float) + (size_t)a.n * (a.n - 1) / 2 * sizeof(uint16_t);
@@ -767,13 +808,19 @@ dpl_status launch_solve_reg_k(const PixArgs& a, cudaStream_t s) {
     int dev = 0, sms = 0;
     DPL_CUDA_TRY(cudaGetDevice(&dev));
     DPL_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    DPL_CUDA_TRY(cudaFuncSetAttribute(k_solve_reg<K, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const auto kernel = k_solve_reg<K, G, kScale>;
+    DPL_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    DPL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve_reg<K, G>, warps * 32, smem));
+    DPL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem));
     const int64_t resident = (int64_t)std::max(1, per_sm) * std::max(1, sms);
     const int64_t grid = std::min<int64_t>((a.npix + groups - 1) / groups, resident * 8);
-    k_solve_reg<K, G><<<(unsigned)std::max<int64_t>(grid, 1), warps * 32, smem, s>>>(a);
+    kernel<<<(unsigned)std::max<int64_t>(grid, 1), warps * 32, smem, s>>>(a);
     return check_launch("k_solve_reg");
+}
+
+template <int K, int G>
+dpl_status launch_solve_reg_k(const PixArgs& a, cudaStream_t s) {
+    return a.ill_list ? launch_solve_reg_kl<K, G, true>(a, s) : launch_solve_reg_kl<K, G, false>(a, s);
 }
 
 }  // namespace dpl
