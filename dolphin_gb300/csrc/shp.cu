@@ -649,8 +649,7 @@ extern "C" dpl_status dpl_shp_glrt(const float* mean, const float* var, int64_t 
 }
 
 size_t dpl::ks_workspace_size(int64_t nslc, int64_t rows, int64_t cols) {
-    return 256 + align_up((size_t)(2 * (nslc + 1)) * sizeof(int), 256) +
-           align_up((size_t)nslc * rows * cols * sizeof(float), 256);
+    return align_up((size_t)nslc * rows * cols * sizeof(float), 256);
 }
 
 // shp/_ks.py:221-239: distances from 0.01 in steps of 0.001, the first whose Kolmogorov

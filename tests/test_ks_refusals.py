@@ -20,3 +20,8 @@ def test_window_too_large(cutoff, is_sorted):
     st = lib.dpl_shp_ks(p, n, rows, cols, hy, hx, 1, 1, cutoff, is_sorted, p, p, size, None)
     assert st == UNSUPPORTED
     assert b"window too large" in lib.dpl_last_error_message()
+
+
+@pytest.mark.parametrize("n,rows,cols", [(1, 1, 1), (20, 37, 41), (64, 512, 512)])
+def test_workspace_holds_the_sorted_samples_only(n, rows, cols):
+    assert _lib.load().dpl_shp_ks_workspace_size(n, rows, cols) == -(-4 * n * rows * cols // 256) * 256
