@@ -149,12 +149,6 @@ namespace dpl {
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t row_mask(const PixArgs& a, int64_t p, int wa, int wx, int lane) {
     const uint64_t full = wx >= 64 ? ~0ull : ((1ull << wx) - 1ull);
-    if (a.nb_bits) {
-        const uint32_t* w = a.nb_bits + ((p * (2 * a.hy + 1) + wa) * a.wpr);
-        uint64_t m = w[0];
-        if (a.wpr > 1) m |= (uint64_t)w[1] << 32;
-        return m & full;
-    }
     if (a.nb_u8) {
         const uint8_t* b = a.nb_u8 + (p * (2 * a.hy + 1) + wa) * wx;
         uint32_t lo = __ballot_sync(0xffffffffu, lane < wx && b[lane] != 0);

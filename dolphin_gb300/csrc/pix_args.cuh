@@ -57,8 +57,6 @@ struct PixArgs {
     size_t off_C, off_G, off_S, off_v, off_d, off_piv, warp_bytes;
     const cfloat* zt;        // (rows, cols, n) masked, pixel-major
     const uint8_t* nb_u8;    // (out_rows, out_cols, wy, wx) or null
-    const uint32_t* nb_bits; // (out_rows, out_cols, wy, wpr) or null
-    int wpr;
     const cfloat* Cin;       // solve-only input: (npix, n, n)
     const cfloat* vstart;    // optional EMI starting vectors (npix, n); plain start when null
     int16_t* iters;          // optional: eigen-iterations used per pixel (npix)
