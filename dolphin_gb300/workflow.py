@@ -424,9 +424,11 @@ def run_wrapped_phase_single(slc_stack, *, half_window, strides=None, first_real
         torch.cuda.current_stream().wait_stream(side)
         while len(_LOOP_GRAPHS) >= _LOOP_GRAPHS_MAX:
             _LOOP_GRAPHS.pop(next(iter(_LOOP_GRAPHS)))
-        _LOOP_GRAPHS[key] = (static_in, g, calls, captured)
+        # every tensor that the graph writes and that is not its own: the int32 counts are in
+        # none of the results
+        _LOOP_GRAPHS[key] = (static_in, rasters, g, calls, captured)
     else:
-        static_in, g, calls, out = entry
+        static_in, _rasters, g, calls, out = entry
         for dst, src in zip(static_in, inputs):
             if dst is not None:
                 dst.copy_(src)
@@ -436,7 +438,8 @@ def run_wrapped_phase_single(slc_stack, *, half_window, strides=None, first_real
 
 
 # Captured block loops (run_wrapped_phase_single(graph=True)), oldest first: the input
-# buffers, the graph, its phase-linking calls (params, workspace) and its outputs.
+# buffers, the rasters that it writes, the graph, its phase-linking calls (params,
+# workspace) and its outputs.
 _LOOP_GRAPHS: dict = {}
 _LOOP_GRAPHS_MAX = 4
 
