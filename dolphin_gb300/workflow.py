@@ -337,7 +337,7 @@ def run_wrapped_phase_single(slc_stack, *, half_window, strides=None, first_real
     blocks runs eagerly on the graph's own input buffers and captures the loop; later
     such calls copy their inputs into those buffers and replay it (one launch from the
     host), then check every block's phase-linking status in order.  The results are
-    copies, the same as the eager loop's.  KS SHPs run eagerly."""
+    copies, the same as the eager loop's."""
     torch = D.require_cuda()
     hw = _yx(half_window, HalfWindow)
     st = _yx(strides if strides is not None else (1, 1), Strides)
@@ -400,8 +400,7 @@ def run_wrapped_phase_single(slc_stack, *, half_window, strides=None, first_real
 
     rasters = (pl, crlb, clos, comp, disp, tcoh, counts, eig, est)
     inputs = (stack, nodata, psm, mean, var)
-    # the KS test copies a host table per call, which a graph cannot replay: eager
-    if not graph or method == ShpMethod.KS:
+    if not graph:
         with deferred_checks():
             return loop(inputs, rasters)
     key = (str(dev), n, rows, cols, hw, st, first_real_slc_idx, output_reference_idx, compressed_reference_idx,
