@@ -8,13 +8,18 @@
 // from shared memory for B^2 complex products.  The window's rows, contiguous in the
 // pixel-major stack, are staged with cp.async one row ahead.
 //
-// Bound by the FP32 pipe: six operations per complex product (a product, a fused
-// multiply-add and an addition per component, the rounding and the order of
-// warp_covariance, so that both give the same sums bit for bit).  A thread per matrix row
-// over all 32 columns, as in warp_covariance, computes 1024 products per sample where
-// N = 21 needs 231; the blocks compute 252.  512 x 384 outputs, 11 x 23 windows, N = 21:
-// 3.6 ms, 21 T operations/s, 57 % of what the pipe issues (a fully set window row skips the
-// search for set bits and takes two samples per turn: 4.0 ms without).
+// Bound by issue (87 % of the slots, the FP32 pipe 64 %): six operations per complex
+// product, a product, a fused multiply-add and an addition per component, rounded and
+// ordered as in warp_covariance.  Both give the same sums bit for bit, but for the imaginary
+// residues of the diagonal, which are left out here, and, above N = 32, the imaginary parts
+// of rows 32 .. by columns 0 .. 31, which warp_covariance sums as the conjugate pair
+// (warp_residues restores both where the plain form's solver reads the matrices).  A thread
+// per matrix row over all 32 columns, as in warp_covariance, computes 1024 products per
+// sample where N = 21 needs 231; the blocks compute 252.  512 x 384 outputs, 11 x 23
+// windows, N = 21: 3.55 ms, 21 T operations/s (a fully set window row skips the search for
+// set bits and takes two samples per turn: 4.0 ms without).  The whole call against the
+// fused plain form, 200 x 150 outputs: N = 21 0.36 of its time, N = 45 0.26, and with the
+// two passes above N = 49, N = 50 0.27 and N = 64 0.23.
 //
 // Output: planar per pixel and normalised, Cg[p][0 .. N^2): diagonal, then (Re, Im) per
 // lower pair, C_ij = numer_ij / sqrt(amp_i amp_j) where that root is > 1e-6, else 0
@@ -109,8 +114,8 @@ __global__ void __launch_bounds__(256, B <= 3 ? 3 : B <= 5 ? 2 : 1) k_cov_simt(c
                 }
                 __syncwarp();  // the row's buffer is refilled by the next stage
             }
-            // the diagonal sums first (the blocks of the first pass hold them all or the
-            // second pass finds them in place): published, then every entry normalised
+            // the diagonal sums first: published (with two passes, those of the other pass are
+            // summed again from global memory), then every entry normalised
             float* amp = reinterpret_cast<float*>(buf);
             if (first == 0 && a.counts && lane == 0) a.counts[p] = count;
             if (active && bi == bj) {

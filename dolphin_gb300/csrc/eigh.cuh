@@ -4,7 +4,7 @@
 // The reference iterates at most 49 times and returns the last iterate, with no flag
 // (phase_link/_eigenvalues.py:194-202).  Where the two eigenvalues nearest the target
 // are close, that iterate is still a mix of their eigenvectors.  Here such pixels are
-// listed by the solvers and solved again, one warp per pixel:
+// listed by the solvers and solved again, by one, two or four warps per pixel:
 //   EMI: |Gamma| (+ beta I, zero threshold) + 1e-6 I is inverted in double precision
 //        (the symmetric sweep operator on its lower triangle), A = |Gamma|^{-1} o C,
 //        and the eigenvector is the one whose eigenvalue is nearest the inverse
@@ -30,13 +30,14 @@ constexpr int kEighSmallN = 16;  // up to here one or two warps per pixel, above
 // mostly short, so the kernel's time is a pixel's latency, not its arithmetic: the phases
 // that have n^2 / 2 independent elements are spread over the CTA's threads, and the FP64
 // pipe, which takes 64 cycles for any warp instruction and has one unit per quarter of the
-// SM, is used in all four quarters.  One warp per pixel, each walking the triangles by
-// division-free row steps, took 483 us for 244 pixels at N = 45 and 389 us for 1882 at
-// N = 30; four warps and a table of the triangle take 181 and 250 us (two: 222 and 239).
-// At N <= 16 a second warp brings 3 pixels of N = 10 from 37 to 30 us (45 before), but
-// 14839 pixels of N = 15, where the SM's issue slots are the limit, from 279 to 490 us:
-// k_eigh_small takes one warp per pixel (274 us; 311 before) once the list is longer than
-// the grid.
+// SM, is used in all four quarters.  244 pixels at N = 45 and 1882 at N = 30 take 181 and
+// 250 us with four warps and a table of the triangle (two warps: 222 and 239; one warp that
+// walks the triangles by division-free row steps: 483 and 389).  At N <= 16 a second warp
+// brings 3 pixels of N = 10 from 37 to 30 us, but 14839 pixels of N = 15, where the SM's
+// issue slots are the limit, from 279 to 490 us: k_eigh_small takes one warp per pixel
+// (274 us) once the list is longer than the grid.  Between N = 17 and 28 the two kernels
+// lie close: the small one takes 2 to 8 % off a whole call with long lists (400 x 400
+// pixels, EVD) and adds up to 3 % to one with short lists (64 x 64).
 template <int W>
 struct EighCta {
     static constexpr int T = 32 * W;

@@ -43,12 +43,13 @@ __device__ __forceinline__ int clamp_start_i(int center, int half, int size, int
 constexpr int kPrepPix = 64;
 inline size_t prep_smem(int n) { return (size_t)kPrepPix * (n | 1) * sizeof(cfloat); }
 
-// HBM-bound by its bytes (8 N in, 8 N + 5 out per pixel).  A tile of 64 pixels is
+// Bound by the latency of its loads and the barriers between its phases: 4.3 TB/s of its
+// bytes (8 N in, 8 N + 5 out per pixel), 64 % of the copy rate.  A tile of 64 pixels is
 // transposed through shared memory at an odd pitch (conflict-free both ways); NaNs and the
 // per-SLC "has a sample" bits are found in the loading loop, where a warp holds one SLC's
-// samples, and only a wanted amplitude mean walks the dates of a pixel.  (The walk for
-// every pixel, by a quarter of the threads and with the magnitudes: 1034 x 1046 pixels at
-// N = 30, 188 us, 123 us now; 1536 x 2304 at N = 21, 445 us, 295 us now.)
+// samples, and only a wanted amplitude mean walks the dates of a pixel.  1034 x 1046
+// pixels at N = 30: 123 us, 1536 x 2304 at N = 21: 295 us (a walk for every pixel, by a
+// quarter of the threads and with the magnitudes: 188 and 445 us).
 __global__ void __launch_bounds__(256) k_prep(const cfloat* __restrict__ slc, int n, int64_t npix,
                                               const uint8_t* __restrict__ nodata_in,
                                               const uint8_t* __restrict__ ps_in, int mask_input_ps,
@@ -591,7 +592,8 @@ struct PostArgs {
 };
 
 
-// HBM-bound by its bytes (12 N in, 12 N out per pixel).  A tile of kPostPix pixels'
+// Bound by the latency of its loads at half of the issue slots: 4.3 TB/s of its bytes (12 N
+// in, 12 N out per pixel), 64 % of the copy rate.  A tile of kPostPix pixels'
 // eigenvectors and CRLBs comes in as the contiguous block it is and leaves by planes
 // through shared memory (odd pitch), 256 / kPostPix threads per pixel; kDirect: a thread
 // per pixel reads its own rows, as short as a sector or two.  The tile by depth, from
@@ -890,10 +892,7 @@ static dpl_status launch_pixel(PixArgs& a, cudaStream_t s, int* fb = nullptr, in
     return launch_pixel_pass<MODE, true>(b, s);
 }
 
-// Tensor-core covariance: fills `Cg` (npix x n*n planar floats).
-// Tile, pass and shared-memory plan of the tensor-core covariance.  False if the
-// shape does not fit (then the plain SIMT form is used).
-// Shared-memory carve of the covariance kernel for nst operand stages, sized for up to
+// Shared-memory carve of the tensor-core covariance for nst operand stages, sized for up to
 // n SLCs, kpad region samples and npass passes (a batch carves once for all its items).
 static void tc_carve(TcArgs& a, int nst, int n, int kpad, int kwords, int npass, bool tf32) {
     size_t o = 0;
@@ -915,6 +914,8 @@ static void tc_carve(TcArgs& a, int nst, int n, int kpad, int kwords, int npass,
     a.smem_bytes = (int)align_up(o, 128) + 1024;  // + alignment slack
 }
 
+// Tile, pass and shared-memory plan of the tensor-core covariance.  False if the shape does
+// not fit (then k_cov_simt and the register solver, or the plain form: pl_finish).
 static bool tc_configure(TcArgs& a, int n, int rows, int cols, int hy, int hx, int sy, int sx, bool tf32 = false) {
     a.n = n;
     a.rows = rows;
@@ -950,6 +951,7 @@ static bool tc_configure(TcArgs& a, int n, int rows, int cols, int hy, int hx, i
     return a.nst >= 2 && a.smem_bytes <= 227 * 1024 && raw <= 2 * (size_t)kTcStageBytes;
 }
 
+// Tensor-core covariance: fills `Cg` (npix x n*n planar floats).
 static dpl_status launch_cov_tc(int n, int rows, int cols, int hy, int hx, int sy, int sx, const cfloat* zt,
                                 const uint8_t* nb_u8, float* Cg, int32_t* counts,
                                 int* status, cudaStream_t s, bool tf32 = false) {

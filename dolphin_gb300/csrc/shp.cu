@@ -13,9 +13,9 @@
 // where the distance to the interval's end is within 5e-7 of it, the decision is taken in
 // double precision on nslc * log1p((s1 - s2)^2 / (4 s1 s2)) (algebraically equal, no
 // cancellation), so every mask bit is the exact comparison on the float32 scale^2.  Few
-// dates (c > 64) compare the two sides, within 2e-6 likewise.  Scales whose products would overflow float32 and thresholds
-// outside the usual range take the statistic with its logarithms (glrt_test), refined
-// in the same way where its rounding could reach the cutoff.
+// dates (c > 64) compare the two sides, within 2e-6 likewise.  Scales whose products would
+// overflow float32 and thresholds outside the usual range take the statistic with its
+// logarithms (glrt_test), refined in the same way where its rounding could reach the cutoff.
 //
 // KS (shp/_ks.py:22-239): amplitudes are sorted per pixel (NaN last, like np.sort).  The
 // reference walks the two-sample merge of each (pixel, neighbour) pair and rejects it
@@ -425,9 +425,9 @@ __device__ __noinline__ bool ks_walk(const float* x1, const float* x2, int n, co
 // only for t < n - d, so the bounds pair up: x2[s + d] > low[s], x2[s] < high[s] for
 // s < ns = n - d, NS being ns rounded up to a multiple of 4.  The samples of a pixel are
 // contiguous in shared memory (immediate offsets), at an odd pitch (consecutive pixels
-// fall into different banks).  Issue-bound (63 % of issue slots): 512 x 512 pixels, 20
-// dates, 11 x 23 windows, 313 us; a merge walk per thread, divergent and with bank
-// conflicts, took 3949 us.
+// fall into different banks).  Bound by issue (71 % of the slots, 61 % of them for loads
+// from shared memory) at 15 warps per SM: 512 x 512 pixels, 20 dates, 11 x 23 windows, 313
+// us (a merge walk per thread, divergent and with bank conflicts: 3949 us).
 template <int NS>
 __global__ void __launch_bounds__(256) k_ks(const __grid_constant__ KsArgs a) {
     extern __shared__ float samp[];  // sorted samples [pixel][np], then the mask bits

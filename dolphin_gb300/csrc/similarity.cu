@@ -21,7 +21,7 @@
 //                The circle's K similarities of a pixel thus sit in the registers of its
 //                group.  The maximum is a group reduction.  For the median the K keys
 //                (order-preserving integers) go through the stage buffer just consumed to
-//                LP = 4 .. 16 lanes per pixel, without the square's corners and the idle
+//                LP = 2 .. 32 lanes per pixel, without the square's corners and the idle
 //                lanes, so that a warp selects for as many pixels at once as fit; each
 //                step of the selection is one group-wide count (redux.sync) around an
 //                interpolated pivot.  The pixel itself (which
@@ -166,8 +166,8 @@ __device__ __forceinline__ float sim_phase(const SimPrepArgs& a, int t, int64_t 
 // exp(i angle z), and z's components added to the sums of nan_to_num(z).  In the ordinary
 // range z / |z|, the reciprocal root refined by one Newton step (components to 2e-7 of
 // their own size); zeros, NaN, infinities and extreme magnitudes by way of the angle.
-// (By way of the angle throughout, the two functions' instructions bounded k_sim_prep:
-// 30 layers of 1400 x 1500 pixels 230 us, 142 us now, 7.1 TB/s.)
+// 30 layers of 1400 x 1500 pixels: 142 us, 7.1 TB/s (by way of the angle throughout, the
+// two functions' instructions bound k_sim_prep: 230 us).
 __device__ __forceinline__ float2 sim_phasor(float2 z, float& sre, float& sim) {
     const float s = fmaf(z.x, z.x, z.y * z.y);
     float2 u;

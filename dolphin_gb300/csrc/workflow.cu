@@ -32,8 +32,8 @@ struct Nodata {
 };
 
 // Compared in the raster's type: in double (as the reference's promotion does, with the
-// same outcome) the 25 comparisons of a 5 x 5 square ran at the FP64 rate: 27 us for a
-// 512 x 512 raster, 5.7 us now.
+// same outcome) the 25 comparisons of a 5 x 5 square run at the FP64 rate: 27 us for a
+// 512 x 512 raster instead of 5.7.
 template <class T>
 __global__ void __launch_bounds__(256) k_grow_nodata(const T* __restrict__ in, T* __restrict__ out, int rows, int cols,
                                                       Nodata<T> nodata, int n) {
